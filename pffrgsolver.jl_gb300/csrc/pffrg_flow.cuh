@@ -14,9 +14,8 @@
 //   wave 0   every subdomain evaluates its first five nodes (the 3-point and
 //            the 5-point Simpson sums) and takes the first convergence test;
 //   wave k   the 2^(k+1) new nodes of every subdomain still refining are cut
-//            into chunks of at most kChunk nodes; eval_kernel spreads the
-//            chunks over the whole GPU and writes one partial node sum per
-//            chunk; decide_kernel sums a subdomain's partials in node order,
+//            into chunks (cut_level); eval_kernel spreads the chunks over the
+//            whole GPU and writes one partial node sum per chunk; decide_kernel sums a subdomain's partials in node order,
 //            forms the next Simpson sum and the Richardson value, takes the
 //            reference's test (||R - S|| < atol or relative < rtol, or
 //            n > 2^20) and either stores the result or queues the next level;
@@ -775,34 +774,54 @@ struct Team {
 // ---------------------------------------------------------------------------
 // wave workspace (device scratch of a pass; one block carved into arrays)
 // ---------------------------------------------------------------------------
-constexpr int kChunk = 32;      // nodes per chunk
-// chunks per subdomain and level (bigger levels use bigger chunks): the deepest subdomains set the
-// length of a pass, so their levels are spread over up to 256 teams (measured on the pyrochlore
-// L = 6 two-loop state: 7 % faster than 64 chunks; 1024 gave the same as 256)
+// The coarse cut of a level of n new nodes: chunks of 32 nodes, at most 256 chunks per subdomain (bigger
+// levels use bigger chunks).  The chunk queue's capacity is counted in coarse chunks.
+constexpr int kChunk = 32;
 constexpr int kMaxChunks = 256;
 
-// Queue the next level (n new nodes) of subdomain sub into wave parity `par`.
-__device__ __forceinline__ void enqueue(WaveSpace& Wsp, int par, int sub, long long n) {
-    long long nch = (n + kChunk - 1) / kChunk;
-    if (nch > kMaxChunks) nch = kMaxChunks;
-    const long long per = (n + nch - 1) / nch;
-    nch = (n + per - 1) / per;
-    const int base = atomicAdd(&Wsp.counters[par], (int)nch);
-    if (base + nch > Wsp.qcap) {
-        atomicOr(&Wsp.counters[4], 1);
-        Wsp.subs[sub].n = 0;
-        return;
+// How the subdomains of a level are cut.  All subdomains refining at one level have the same number n of
+// new nodes (4 at the first level, doubled at each), so a chunk index is (subdomain, part) arithmetic and
+// no queue of chunk records is written or read.
+struct LevelCut {
+    int nact;    // subdomains cut (fewer than are active only after an overflow)
+    int coarse;  // coarse chunks per subdomain
+    int chunks;  // chunks per subdomain (a multiple of coarse)
+    int per;     // nodes per chunk
+    bool overflow;
+};
+
+// Few active subdomains leave most teams without a coarse chunk, and a level then lasts as long as one
+// team takes for 32 nodes one after another (square L = 3 FP64: 93, 166, 308 and 570 us for chunks of 4,
+// 8, 16 and 32 nodes; kagome L = 8 FP64: 10 ms for every level).  Chunks are therefore halved, down to one
+// batch of nodes, while the level still has fewer chunks than `teams`, about twice the teams that the GPU
+// holds at once; larger levels keep the coarse cut, whose partial sums cost least.
+__host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, int batch, int teams) {
+    LevelCut k;
+    const int per0 = n <= (long long)kChunk * kMaxChunks ? (int)(n < kChunk ? n : kChunk) : (int)(n / kMaxChunks);
+    k.coarse = (int)(n / per0);
+    k.overflow = (long long)nact * k.coarse > qcap;
+    k.nact = k.overflow ? qcap / k.coarse : nact;
+    k.per = per0;
+    k.chunks = k.coarse;
+    // the upper half of the partial sums holds the fine chunks' sums of |node values| (fine_abs)
+    const long long most = teams < qcap / 2 ? teams : qcap / 2;
+    while (k.per > batch && 2ll * k.nact * k.chunks <= most) {
+        k.per >>= 1;
+        k.chunks <<= 1;
     }
-    for (int k = 0; k < nch; ++k) {
-        const long long f = k * per;
-        const long long c = (f + per <= n) ? per : n - f;
-        Wsp.queue[par][base + k] = make_int4(sub, (int)f, (int)c, 0);
-    }
-    Wsp.subs[sub].chunk0 = base;
-    Wsp.subs[sub].nchunk = (int)nch;
-    Wsp.subs[sub].n = n;
+    return k;
+}
+
+// per-site sums of |node values| of the fine chunks of a level (FP32 pass of the mixed path): vectors
+// behind the at most qcap / 2 partial sums of such a level
+__device__ __forceinline__ float* fine_abs(const WaveSpace& Wsp, int CNs) {
+    return reinterpret_cast<float*>(Wsp.part + (size_t)(Wsp.qcap - Wsp.qcap / 2) * CNs);
+}
+
+// list subdomain sub for the next level, wave parity par
+__device__ __forceinline__ void enqueue(WaveSpace& Wsp, int par, int sub) {
     const int a = atomicAdd(&Wsp.counters[2 + par], 1);
-    Wsp.active[par][a] = sub;
+    (par ? Wsp.active[1] : Wsp.active[0])[a] = sub;
 }
 
 // the meshes of the node setup (shared memory): FP64 for the FP64 path, float-float pairs for the
@@ -1014,7 +1033,6 @@ __device__ __forceinline__ double team_norm(const double v[C][SPL]) {
 
 // hand a subdomain from the FP32 pass to the FP64 pass (team lane 0)
 __device__ __forceinline__ void hand_off(WaveSpace& Wsp, int sub) {
-    Wsp.subs[sub].n = 0;
     Wsp.esc[atomicAdd(&Wsp.counters[5], 1)] = sub;
 }
 
@@ -1138,7 +1156,6 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
                     const int i = tl + k * T;
                     if (i < Ns) sA[c * Ns + i] = boundary ? c0 * (double)g[0][c][k] + c1 * (double)g[1][c][k] : 0.0;
                 }
-            if (tl == 0) Wsp.subs[sub].n = 0;
             continue;
         }
 #pragma unroll
@@ -1161,8 +1178,7 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
             S.sgn = sgn;
             S.sa = sa_new;
             S.fab = fab;
-            if (done) S.n = 0;
-            else enqueue(Wsp, 1, sub, 4);
+            if (!done) enqueue(Wsp, 1, sub);
         }
     }
     if (A.node_counter && tl == 0) {
@@ -1180,16 +1196,22 @@ template <typename R, int T, int SPL, int C>
 constexpr int eval_min_blocks() { return sizeof(R) == 4 ? (C == 2 && SPL <= 2 ? 4 : 3) : 1; }
 
 template <typename R, int T, int SPL, int C>
-__global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>()) eval_kernel(PassArgs<R> A, WaveSpace Wsp, int par) {
+__global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
+    eval_kernel(PassArgs<R> A, WaveSpace Wsp, int par, long long n) {
     constexpr int NPW = 32 / T;
+    constexpr int NB = BatchOf<T, C, SPL>::NB;
     extern __shared__ __align__(16) unsigned char smem[];
+    const int nactive = Wsp.counters[2 + par];
+    const LevelCut K = cut_level(nactive, n, Wsp.qcap, NB, Wsp.teams);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        // the next level's queue starts empty (its chunks are enqueued by this wave's decide_kernel)
-        Wsp.counters[par ^ 1] = 0;
+        // the next level's list starts empty (this wave's decide_kernel fills it)
         Wsp.counters[2 + (par ^ 1)] = 0;
+        // a level whose coarse chunks exceed the queue's capacity is reported and cut short
+        if (K.overflow) Wsp.counters[4] = 1;
     }
+    const int nchunks = K.nact * K.chunks;
     // blocks without a chunk leave before staging the meshes and rows
-    if ((long long)blockIdx.x * kWarps * NPW >= Wsp.counters[par]) return;
+    if ((long long)blockIdx.x * kWarps * NPW >= nchunks) return;
     load_common<R, T, C, SPL>(A, smem);
     const auto M = setup_mesh(A, smem);  // staged in shared memory by load_common
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1197,31 +1219,27 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>()) 
     Team<R, T, SPL, C> tm = make_team<R, T, SPL, C>(A, smem, M, warp, team, tl);
     const int Ns = A.L.Ns;
     const int jobs = 4 * A.eval + 1;
-    // a level whose chunks overflowed the queue counted them all; only the first qcap were filed
-    const int nchunks = min(Wsp.counters[par], Wsp.qcap);
+    const int* active = par ? Wsp.active[1] : Wsp.active[0];
     const long long nwarps = (long long)gridDim.x * kWarps;
-    constexpr int NB = BatchOf<T, C, SPL>::NB;
     for (long long base = ((long long)blockIdx.x * kWarps + warp) * NPW; base < nchunks; base += nwarps * NPW) {
         const int chunk = (int)(base + team);
         const bool valid = chunk < nchunks;
-        int4 cr = make_int4(0, 0, 0, 0);
+        int first = 0;  // first new node of the chunk
         TaskInfo ti{0, 1, 0, 0, 0};
         double lo = 0, h = 0, sgn = 1;
         typename Team<R, T, SPL, C>::SetupT W(0.0), V(0.0), VP(0.0);
         if (valid) {
-            cr = Wsp.queue[par][chunk];
-            const SubRec S = Wsp.subs[cr.x];
-            ti = task_of(A, cr.x, jobs);
+            const int a = chunk / K.chunks;
+            const int sub = active[a];
+            first = (chunk - a * K.chunks) * K.per;
+            const SubRec S = Wsp.subs[sub];
+            ti = task_of(A, sub, jobs);
             task_freqs(A, M, ti, W, V, VP);
             lo = S.lo;
             sgn = S.sgn;
-            h = 0.5 * (S.hi - S.lo) / (double)S.n;
+            h = 0.5 * (S.hi - S.lo) / (double)n;
         }
-        // the longest chunk of the warp's teams bounds the batch loop
-        int cnt = valid ? cr.z : 0;
-        int mx = cnt;
-#pragma unroll
-        for (int o = T; o < 32; o <<= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
+        const int cnt = valid ? K.per : 0;
         Acc<R> acc[C][SPL];
         R aab[C][SPL];  // FP32 pass of the mixed path: sums of |node values|
 #pragma unroll
@@ -1241,17 +1259,17 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>()) 
                     if constexpr (sizeof(R) == 4) aab[c][k] += fabsf(gv[c][k]);
                 }
         };
-        for (int b = 0; b < mx; b += NB) {
+        for (int b = 0; b < K.per; b += NB) {
             const int nb = max(0, min(NB, cnt - b));
             if (tl < nb) {
-                const long long nd = (long long)cr.y + b + tl;  // 0-based new node of the level
+                const int nd = first + b + tl;  // 0-based new node of the level
                 tm.ts.node[tl].x = sgn * __dadd_rn(lo, __dmul_rn(2.0 * (double)(nd + 1) - 1.0, h));
             }
             __syncwarp();
             tm.eval(ti, W, V, VP, nb, add);
         }
         if constexpr (sizeof(R) == 4) {
-            if (A.esc_mode == 1) {
+            if (A.esc_mode == 1 && K.chunks == K.coarse) {
                 double ad[C][SPL];
 #pragma unroll
                 for (int c = 0; c < C; ++c)
@@ -1270,6 +1288,19 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>()) 
                 const int i = tl + k * T;
                 if (i < Ns) P[c * Ns + i] = (double)acc[c][k].s + (double)acc[c][k].c;
             }
+        if constexpr (sizeof(R) == 4) {
+            if (A.esc_mode == 1 && K.chunks != K.coarse) {
+                // the coarse chunk's norm is formed from its fine chunks' sums by decide_kernel
+                float* Q = fine_abs(Wsp, C * Ns) + (size_t)chunk * C * Ns;
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int k = 0; k < SPL; ++k) {
+                        const int i = tl + k * T;
+                        if (i < Ns) Q[c * Ns + i] = aab[c][k];
+                    }
+            }
+        }
     }
     if (A.node_counter && tl == 0) {
         atomicAdd(A.node_counter, tm.nodes);
@@ -1278,50 +1309,120 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>()) 
 }
 
 // ---- wave k >= 1: per subdomain, next Simpson sum, test, result or next level ----
+// One team per subdomain, or, for subdomains of many chunks, all teams of a block: each sums a part of the
+// chunks and the first team forms the total from their sums in order.
+constexpr int kDecideSplit = 64;  // chunks per subdomain from which a block's teams share them
+
 template <int T, int SPL, int C>
 __global__ void __launch_bounds__(kWarps * 32) decide_kernel(WaveSpace Wsp, int Ns, double atol, double rtol, int par,
-                                                             int esc_mode, double esc_eps) {
+                                                             long long n, int esc_mode, double esc_eps) {
     constexpr int NPW = 32 / T;
+    constexpr int TPB = kWarps * NPW;  // teams per block
+    static_assert(kDecideSplit >= TPB, "every team of a block has a chunk");
+    __shared__ double sh_f[TPB - 1][C * SPL * T];  // sums of all teams but the first
+    __shared__ double sh_a[TPB - 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int team = lane / T, tl = lane % T;
-    const int nact = Wsp.counters[2 + par];
-    const long long nwarps = (long long)gridDim.x * kWarps;
-    for (long long base = ((long long)blockIdx.x * kWarps + warp) * NPW; base < nact; base += nwarps * NPW) {
-        const int a = (int)(base + team);
-        const bool valid = a < nact;
-        const int sub = valid ? Wsp.active[par][a] : 0;
+    const int bteam = warp * NPW + team;
+    const LevelCut K = cut_level(Wsp.counters[2 + par], n, Wsp.qcap, BatchOf<T, C, SPL>::NB, Wsp.teams);
+    const int* active = par ? Wsp.active[1] : Wsp.active[0];
+    const bool split = K.chunks >= kDecideSplit;
+    const int G = split ? TPB : 1, g = split ? bteam : 0;
+    const int step = split ? gridDim.x : gridDim.x * TPB;
+    const int q0 = K.chunks / G * g, q1 = q0 + K.chunks / G;
+    // coarse chunks of this team's share of the |node value| norms
+    const int ca = (K.coarse + G - 1) / G, c0 = min(K.coarse, g * ca), c1 = min(K.coarse, c0 + ca);
+    for (int base = split ? blockIdx.x : blockIdx.x * TPB + warp * NPW; base < K.nact; base += step) {
+        const int a = split ? base : base + team;
+        const bool valid = a < K.nact;
+        const int sub = valid ? active[a] : 0;
         SubRec S;
         if (valid) S = Wsp.subs[sub];
-        else S.n = 1, S.nchunk = 0, S.chunk0 = 0, S.lo = 0, S.hi = 0;
+        else S.lo = 0, S.hi = 0, S.sa = 0, S.fab = 0;
         double* sA = Wsp.stA + (size_t)sub * C * Ns;
         double* sB = Wsp.stB + (size_t)sub * C * Ns;
         double s_old[C][SPL], s_new[C][SPL], f_new[C][SPL];
-        const double h = 0.5 * (S.hi - S.lo) / (double)S.n;
+        const double h = 0.5 * (S.hi - S.lo) / (double)n;
         const double wn = 4.0 * h / 3.0, wo = -2.0 * h / 3.0;
+        const double* part = Wsp.part + (size_t)(valid ? a : 0) * K.chunks * C * Ns;
 #pragma unroll
         for (int c = 0; c < C; ++c)
 #pragma unroll
             for (int k = 0; k < SPL; ++k) {
                 const int i = tl + k * T;
-                s_old[c][k] = s_new[c][k] = f_new[c][k] = 0.0;
+                f_new[c][k] = 0.0;
                 if (!valid || i >= Ns) continue;
                 double f = 0.0;
-                for (int q = 0; q < S.nchunk; ++q) f += Wsp.part[(size_t)(S.chunk0 + q) * C * Ns + c * Ns + i];
+#pragma unroll 4
+                for (int q = q0; q < q1; ++q) f += part[(size_t)q * C * Ns + c * Ns + i];
                 f_new[c][k] = f;
+            }
+        double fa_new = 0.0;
+        if (esc_mode == 1 && K.chunks == K.coarse) {
+            if (valid)
+                for (int q = q0; q < q1; ++q) fa_new += Wsp.part_abs[(size_t)a * K.chunks + q];  // triangle bound
+        } else if (esc_mode == 1) {
+            // the norms of the coarse chunks, from the sums of their fine chunks: the bound (and with it
+            // which subdomains are handed off) does not depend on how a level was cut
+            const int r = K.chunks / K.coarse;
+            const float* Q = fine_abs(Wsp, C * Ns) + (size_t)(valid ? a : 0) * K.chunks * C * Ns;
+            for (int cc = 0; cc < ca; ++cc) {
+                const int q = c0 + cc;
+                double ad[C][SPL];
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int k = 0; k < SPL; ++k) {
+                        const int i = tl + k * T;
+                        float f = 0.f;
+                        if (valid && i < Ns && q < c1)
+                            for (int e = 0; e < r; ++e) f += Q[(size_t)(q * r + e) * C * Ns + c * Ns + i];
+                        ad[c][k] = (double)f;
+                    }
+                fa_new += team_norm<T, SPL, C>(ad);  // every lane of the warp takes part
+            }
+        }
+        if (split) {
+            __syncthreads();  // the sums of the previous subdomain have been read
+            if (bteam > 0) {
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int k = 0; k < SPL; ++k) sh_f[bteam - 1][(c * SPL + k) * T + tl] = f_new[c][k];
+                if (tl == 0) sh_a[bteam - 1] = fa_new;
+            }
+            __syncthreads();
+            if (warp > 0) continue;
+            // the first team adds them in order (the others of its warp only take part in its shuffles)
+#pragma unroll
+            for (int e = 0; e < TPB - 1; ++e) {
+                fa_new += sh_a[e];
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int k = 0; k < SPL; ++k) f_new[c][k] += sh_f[e][(c * SPL + k) * T + tl];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int k = 0; k < SPL; ++k) {
+                const int i = tl + k * T;
+                s_old[c][k] = s_new[c][k] = 0.0;
+                if (!valid || i >= Ns) continue;
                 s_old[c][k] = sA[c * Ns + i];
-                s_new[c][k] = 0.5 * s_old[c][k] + wn * f + wo * sB[c * Ns + i];
+                s_new[c][k] = 0.5 * s_old[c][k] + wn * f_new[c][k] + wo * sB[c * Ns + i];
             }
         int done;
-        double sa_new = 0.0, fa_new = 0.0;
+        double sa_new = 0.0;
         if (esc_mode == 1) {
-            for (int q = 0; q < S.nchunk; ++q) fa_new += Wsp.part_abs[S.chunk0 + q];  // triangle bound
-            const double sa_old = valid ? S.sa : 0.0;
-            sa_new = 0.5 * sa_old + fabs(wn) * fa_new + fabs(wo) * (valid ? S.fab : 0.0);
-            done = simps_decide<T, SPL, C>(s_old, s_new, S.n, atol, rtol, esc_eps, sa_old, sa_new);
+            const double sa_old = S.sa;
+            sa_new = 0.5 * sa_old + fabs(wn) * fa_new + fabs(wo) * S.fab;
+            done = simps_decide<T, SPL, C>(s_old, s_new, n, atol, rtol, esc_eps, sa_old, sa_new);
         } else {
-            done = simps_test<T, SPL, C>(s_old, s_new, S.n, atol, rtol, team, false);
+            done = simps_test<T, SPL, C>(s_old, s_new, n, atol, rtol, team, false);
         }
-        if (!valid) continue;
+        if (!valid || (split && team > 0)) continue;
         if (done == 2) {
             if (tl == 0) hand_off(Wsp, sub);
             continue;
@@ -1339,14 +1440,10 @@ __global__ void __launch_bounds__(kWarps * 32) decide_kernel(WaveSpace Wsp, int 
                     sB[c * Ns + i] = f_new[c][k];
                 }
             }
-        if (tl == 0) {
-            if (done) {
-                Wsp.subs[sub].n = 0;
-            } else {
-                Wsp.subs[sub].sa = sa_new;
-                Wsp.subs[sub].fab = fa_new;
-                enqueue(Wsp, par ^ 1, sub, 2 * S.n);
-            }
+        if (tl == 0 && !done) {
+            Wsp.subs[sub].sa = sa_new;
+            Wsp.subs[sub].fab = fa_new;
+            enqueue(Wsp, par ^ 1, sub);
         }
     }
 }
@@ -1412,6 +1509,7 @@ struct PassLauncher {
         const int teams_per_block = kWarps * NPW;
         // the FP64 pass of the mixed path keeps the count of handed subdomains (counters[5])
         if ((e = cudaMemsetAsync(Wsp.counters, 0, sizeof(int) * (a.esc_mode == 2 ? 5 : 6), st))) return e;
+        Wsp.teams = 2 * 4 * 152 * teams_per_block;  // twice the teams of four blocks per SM
         int g0 = (Wsp.nsub + teams_per_block - 1) / teams_per_block;
         // h_counters[7] counts the kernels this pass launches
         wave0_kernel<R, T, SPL, C><<<g0 < grid_cap ? g0 : grid_cap, kWarps * 32, smem, st>>>(a, Wsp);
@@ -1424,11 +1522,11 @@ struct PassLauncher {
             const int gd = std::max(1, std::min(grid_cap, (Wsp.nsub + teams_per_block - 1) / teams_per_block));
             int par = 1;
             for (int wave = 1; wave <= 21; ++wave) {
-                eval_kernel<R, T, SPL, C><<<grid_cap, kWarps * 32, smem, st>>>(a, Wsp, par);
+                eval_kernel<R, T, SPL, C><<<grid_cap, kWarps * 32, smem, st>>>(a, Wsp, par, 2ll << wave);
                 h_counters[7] += 2;
                 if ((e = cudaGetLastError())) return e;
-                decide_kernel<T, SPL, C><<<gd, kWarps * 32, 0, st>>>(Wsp, a.L.Ns, a.atol, a.rtol, par, a.esc_mode,
-                                                                     a.esc_eps);
+                decide_kernel<T, SPL, C><<<gd, kWarps * 32, 0, st>>>(Wsp, a.L.Ns, a.atol, a.rtol, par, 2ll << wave,
+                                                                     a.esc_mode, a.esc_eps);
                 if ((e = cudaGetLastError())) return e;
                 par ^= 1;
             }
@@ -1444,19 +1542,21 @@ struct PassLauncher {
         for (int wave = 1; wave <= 21; ++wave) {
             if ((e = cudaMemcpyAsync(h_counters, Wsp.counters, sizeof(int) * 5, cudaMemcpyDeviceToHost, st))) return e;
             if ((e = cudaStreamSynchronize(st))) return e;
-            if (h_counters[4]) return cudaErrorLaunchOutOfResources;  // chunk queue overflow
-            const int nchunks = h_counters[par], nact = h_counters[2 + par];
+            const int nact = h_counters[2 + par];
             if (nact == 0) break;
-            // reset the other parity's counters for the next wave's queue
-            if ((e = cudaMemsetAsync(Wsp.counters + (par ^ 1), 0, sizeof(int), st))) return e;
-            if ((e = cudaMemsetAsync(Wsp.counters + 2 + (par ^ 1), 0, sizeof(int), st))) return e;
-            int ge = (nchunks + teams_per_block - 1) / teams_per_block;
-            eval_kernel<R, T, SPL, C><<<ge < grid_cap ? ge : grid_cap, kWarps * 32, smem, st>>>(a, Wsp, par);
+            const LevelCut K = cut_level(nact, 2ll << wave, Wsp.qcap, BatchOf<T, C, SPL>::NB, Wsp.teams);
+            if (K.overflow) {  // chunk queue overflow
+                h_counters[4] = 1;
+                return cudaErrorLaunchOutOfResources;
+            }
+            int ge = (K.nact * K.chunks + teams_per_block - 1) / teams_per_block;
+            eval_kernel<R, T, SPL, C><<<ge < grid_cap ? ge : grid_cap, kWarps * 32, smem, st>>>(a, Wsp, par, 2ll << wave);
             h_counters[7] += 2;
             if ((e = cudaGetLastError())) return e;
             int gd = (nact + teams_per_block - 1) / teams_per_block;
             decide_kernel<T, SPL, C><<<gd < grid_cap ? gd : grid_cap, kWarps * 32, 0, st>>>(Wsp, a.L.Ns, a.atol, a.rtol,
-                                                                                           par, a.esc_mode, a.esc_eps);
+                                                                                           par, 2ll << wave, a.esc_mode,
+                                                                                           a.esc_eps);
             if ((e = cudaGetLastError())) return e;
             par ^= 1;
         }

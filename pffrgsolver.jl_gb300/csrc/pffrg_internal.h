@@ -66,13 +66,10 @@ struct PassArgs {
 };
 
 // Scratch of one pass of the level-synchronous quadrature: one record and two state
-// vectors per Simpson subdomain, the chunk queues of the current and next level, and one
-// partial node sum per chunk.  Carved out of one device block.
+// vectors per Simpson subdomain, the lists of the subdomains refining at the current and the
+// next level, and one partial node sum per chunk.  Carved out of one device block.
 struct SubRec {
     double lo, hi, sgn;
-    long long n;  // new nodes of the pending level (0: finished)
-    int chunk0;   // first chunk of the pending level in the wave queue
-    int nchunk;
     double sa;    // FP32 pass: bound of |weights| x |node values| of the last Simpson sum (norm)
     double fab;   // and of the last level's new nodes
 };
@@ -81,13 +78,13 @@ struct WaveSpace {
     SubRec* subs;    // [nsub]
     double* stA;     // [nsub][C Ns]: Simpson sum of the last level, then the result
     double* stB;     // [nsub][C Ns]: node sum of the last level's new nodes
-    int4* queue[2];  // chunk records (sub, first node, count, -) of the current / next level
-    int* active[2];  // subdomains with chunks in the current / next level
+    int* active[2];  // subdomains refining at the current / next level
     double* part;    // [qcap][C Ns] chunk partial node sums
     double* part_abs;  // [qcap] FP32 pass: norm of the chunk's sums of |node values|
     int* esc;        // [nsub] subdomains handed from the FP32 pass to the FP64 pass
-    int* counters;   // [0..1] chunks, [2..3] active subdomains per parity, [4] queue overflow, [5] handed
+    int* counters;   // [2..3] active subdomains per parity, [4] queue overflow, [5] handed
     int nsub, qcap;
+    int teams;       // chunks that a level with few subdomains is cut into (cut_level)
 };
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -140,7 +137,7 @@ inline void append_inverse_spacings(std::vector<double>& h, int Nsig, int NO, in
 // bytes of the wave workspace for nsub subdomains, C components on Ns sites and qcap chunks
 inline size_t wave_space_bytes(long long nsub, int Ns, long long qcap, int C) {
     const size_t vec = sizeof(double) * C * (size_t)Ns;
-    return align256(sizeof(SubRec) * nsub) + 2 * align256(vec * nsub) + 2 * align256(sizeof(int4) * qcap) +
+    return align256(sizeof(SubRec) * nsub) + 2 * align256(vec * nsub) +
            2 * align256(sizeof(int) * nsub) + align256(vec * qcap) + align256(sizeof(double) * qcap) +
            align256(sizeof(int) * nsub) + align256(sizeof(int) * 8);
 }
@@ -154,10 +151,6 @@ inline void wave_space_carve(WaveSpace& W, void* base, long long nsub, int Ns, l
     p += align256(vec * nsub);
     W.stB = reinterpret_cast<double*>(p);
     p += align256(vec * nsub);
-    for (int k = 0; k < 2; ++k) {
-        W.queue[k] = reinterpret_cast<int4*>(p);
-        p += align256(sizeof(int4) * qcap);
-    }
     for (int k = 0; k < 2; ++k) {
         W.active[k] = reinterpret_cast<int*>(p);
         p += align256(sizeof(int) * nsub);

@@ -120,26 +120,45 @@ struct Param {
     R wl, wu;
 };
 
+// Comparisons of the interval searches and buffer switches.  An FP64 compare goes through the FP64
+// pipe, which takes 16 cycles for a warp here (two lanes per clock and SM) and is what bounds the
+// FP64 kernels; non-negative doubles order like their bits, so the FP64 overloads compare integers.
+__device__ __forceinline__ bool is_neg(float x) { return x < 0.f; }
+__device__ __forceinline__ bool is_neg(double x) {  // x < 0 (false for -0)
+    const long long k = __double_as_longlong(x);
+    return k < 0 && k != (long long)0x8000000000000000ull;
+}
+// a < b for a, b >= 0
+__device__ __forceinline__ bool less_nonneg(float a, float b) { return a < b; }
+__device__ __forceinline__ bool less_nonneg(double a, double b) {
+    return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ bool is_nan(float x) { return x != x; }
+__device__ __forceinline__ bool is_nan(double x) {
+    return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+
 // get_indices + get_param (param.jl:26-87) with a binary search that returns
 // the same pair as the reference's linear scan: hi = first k with x[k] >= val.
+// (val and the mesh are not negative)
 template <typename R>
 __device__ __forceinline__ Param<R> get_param(R val, const R* x, const R* ix, int n) {
     Param<R> p;
-    if (val >= x[n - 1]) {
+    const bool nan = is_nan(val);  // NaN: the linear scan stops at the first entry
+    if (!nan && !less_nonneg(val, x[n - 1])) {
         p.lo = p.hi = n - 1;
         p.wl = (R)1;
         p.wu = (R)0;
         return p;
     }
-    int lo = 0, hi = n - 1;
-    if (!(val == val)) hi = 0;  // NaN: the linear scan stops at the first entry
+    int lo = 0, hi = nan ? 0 : n - 1;
     while (lo < hi) {
         int mid = (lo + hi) >> 1;
-        if (x[mid] >= val) hi = mid;
+        if (!less_nonneg(x[mid], val)) hi = mid;
         else lo = mid + 1;
     }
     p.hi = lo;
-    p.lo = (val < x[lo]) ? lo - 1 : lo;
+    p.lo = (!nan && less_nonneg(val, x[lo])) ? lo - 1 : lo;
     if (p.lo < 0) p.lo = 0;
     if (p.lo < p.hi) {
         R d = ix[p.lo];
@@ -175,23 +194,23 @@ __device__ __forceinline__ void make_plan(Plan<R>& P, int chan, S w, S v, S vp, 
                                           int Nn) {
     bool ex = false, mp = false, smn = false, sm = false, sn = false;
     if (chan == 0) {  // get_buffer_s (buffer.jl:87-124)
-        if (w < (S)0) { w = -w; ex = !ex; }
-        if (v < (S)0) { v = -v; ex = !ex; mp = !mp; sm = !sm; }
-        if (vp < (S)0) { vp = -vp; mp = !mp; sn = !sn; }
+        if (is_neg(w)) { w = -w; ex = !ex; }
+        if (is_neg(v)) { v = -v; ex = !ex; mp = !mp; sm = !sm; }
+        if (is_neg(vp)) { vp = -vp; mp = !mp; sn = !sn; }
     } else if (chan == 1) {  // get_buffer_t (buffer.jl:126-160)
-        if (w < (S)0) { w = -w; smn = !smn; }
-        if (v < (S)0) { v = -v; sm = !sm; }
-        if (vp < (S)0) { vp = -vp; sn = !sn; }
+        if (is_neg(w)) { w = -w; smn = !smn; }
+        if (is_neg(v)) { v = -v; sm = !sm; }
+        if (is_neg(vp)) { vp = -vp; sn = !sn; }
     } else {  // get_buffer_u (buffer.jl:162-199)
-        if (w < (S)0) { w = -w; ex = !ex; smn = !smn; }
-        if (v < (S)0) { v = -v; ex = !ex; mp = !mp; sn = !sn; }
-        if (vp < (S)0) { vp = -vp; mp = !mp; sn = !sn; }
+        if (is_neg(w)) { w = -w; ex = !ex; smn = !smn; }
+        if (is_neg(v)) { v = -v; ex = !ex; mp = !mp; sn = !sn; }
+        if (is_neg(vp)) { vp = -vp; mp = !mp; sn = !sn; }
     }
     const S* Om = chan == 1 ? M.Ot : M.Os;
     const S* iOm = chan == 1 ? M.iOt : M.iOs;
     const S* nu = chan == 1 ? M.nt : M.ns;
     const S* inu = chan == 1 ? M.int_ : M.ins;
-    if (Om[NO - 1] < fabs(w)) {  // get_buffer (buffer.jl:51-84): beyond the bosonic mesh
+    if (!is_nan(w) && less_nonneg(Om[NO - 1], w)) {  // get_buffer (buffer.jl:51-84): beyond the bosonic mesh
         P.kernel = 0;
         return;
     }
@@ -200,8 +219,8 @@ __device__ __forceinline__ void make_plan(Plan<R>& P, int chan, S w, S v, S vp, 
     P.src_ch = (chan == 1) ? 1 : ((chan == 0) == mp ? 2 : 0);
     P.sgn_d = ((sm ? -1 : 1) * (sn ? -1 : 1)) < 0 ? (R)-1 : (R)1;
     const Param<S> p1 = get_param(w, Om, iOm, NO);
-    const bool vin = !(nu[Nn - 1] < fabs(v));
-    const bool vpin = !(nu[Nn - 1] < fabs(vp));
+    const bool vin = is_nan(v) || !less_nonneg(nu[Nn - 1], v);
+    const bool vpin = is_nan(vp) || !less_nonneg(nu[Nn - 1], vp);
     if (!vin && !vpin) {
         P.kernel = 1;
         P.w[0] = (R)(p1.wl);
@@ -275,8 +294,8 @@ __device__ __forceinline__ R plan_read(const Plan<R>& P, const R* __restrict__ q
 // apply_flags_su2 (action_su2.jl:73-92) for C = 2 and apply_flags_u1_dm
 // (action_u1_dm.jl:80-118) for C = 6: the component a plan reads for component
 // c (xx, zz, DM, dd, zd, dz for u1-dm) and the sign of its contribution
-template <typename R>
-__device__ __forceinline__ int comp_read(const Plan<R>& P, int C, int c, R& sgn) {
+template <typename R, typename PL>
+__device__ __forceinline__ int comp_read(const PL& P, int C, int c, R& sgn) {
     if (C == 2) {
         sgn = c == 1 ? P.sgn_d : (R)1;
         return c;
@@ -609,6 +628,274 @@ __device__ __forceinline__ float G_full_s(float s, float L, float w) {
         return 1.f / den;
     }
     return 0.f;
+}
+
+// ---------------------------------------------------------------------------
+// Node setup of the quadrature passes: the plans of a node live in shared memory and every lane of
+// the team reads them, so a plan keeps only the corners that count, ready to use.
+// ---------------------------------------------------------------------------
+template <typename R>
+struct NodePlan {
+    int64_t base;  // offset of the kernel read, component 0
+    int nc;        // corners (0: nothing is read)
+    int exch;
+    int flags;     // bit 0: sgn_μν, bit 1: sgn_μ, bit 2: sgn_ν, bit 3: two bosonic corners
+    R sgn_d;
+    R w[8];
+    int off[8];
+};
+
+// FP64 mesh block staged in shared memory: values, then inverse spacings, [σ | Ωs | νs | Ωt | νt] each
+struct MeshD {
+    const double* x;
+    const double* inv;
+    int Nsig, NO, Nn;
+    __device__ __forceinline__ int sig() const { return 0; }
+    __device__ __forceinline__ int Os() const { return Nsig; }
+    __device__ __forceinline__ int ns() const { return Nsig + NO; }
+    __device__ __forceinline__ int Ot() const { return Nsig + NO + Nn; }
+    __device__ __forceinline__ int nt() const { return Nsig + 2 * NO + Nn; }
+    __device__ __forceinline__ double at(int o, int k) const { return x[o + k]; }
+};
+
+__device__ __forceinline__ MeshD mesh_view_d(const double* block, int Nsig, int NO, int Nn) {
+    return MeshD{block, block + Nsig + 2 * NO + 2 * Nn, Nsig, NO, Nn};
+}
+
+__device__ __forceinline__ bool is_neg(FF x) { return x < 0.f; }
+__device__ __forceinline__ bool beyond(FF last, FF x) { return last < x; }
+__device__ __forceinline__ bool beyond(double last, double x) { return !is_nan(x) && less_nonneg(last, x); }
+__device__ __forceinline__ Param<float> find(FF x, const MeshFF& M, int o, int n) { return get_param_ff(x, M, o, n); }
+__device__ __forceinline__ Param<double> find(double x, const MeshD& M, int o, int n) {
+    return get_param(x, M.x + o, M.inv + o, n);
+}
+
+// The plan of one buffer (same sign folding, kernel choice and corner order as make_plan).  Corners
+// of an argument that lies exactly on a mesh point, whose second weight is zero, are left out: the
+// bubbles read their own channel at the task's mesh frequencies, where two corners of eight remain.
+// q0: offset of the first kernel of the s channel.  Returns the kernel (0 none, 1 q1, ..., 4 q3).
+template <typename R, typename S, typename MV>
+__device__ __forceinline__ int build_plan(NodePlan<R>& P, int chan, S w, S v, S vp, const MV& M, int Ns,
+                                          int64_t q0) {
+    const bool nw = is_neg(w), nv = is_neg(v), np = is_neg(vp);
+    if (nw) w = -w;
+    if (nv) v = -v;
+    if (np) vp = -vp;
+    // buffer.jl:87-199: exchange, s <-> u mapping and the three signs of a folded argument
+    const bool ex = chan == 1 ? false : nw != nv;
+    const bool mp = chan != 1 && nv != np;
+    const bool smn = chan != 0 && nw;
+    const bool sm = chan != 2 && nv;
+    const bool sn = chan == 2 ? nv != np : np;
+    const int NO = M.NO, Nn = M.Nn;
+    const int oO = chan == 1 ? M.Ot() : M.Os();
+    const int on = chan == 1 ? M.nt() : M.ns();
+    if (beyond(M.at(oO, NO - 1), w)) {  // get_buffer (buffer.jl:51-84): beyond the bosonic mesh
+        P.nc = 0;
+        return 0;
+    }
+    const S last = M.at(on, Nn - 1);
+    const bool vin = !beyond(last, v), vpin = !beyond(last, vp);
+    const int kernel = vin ? (vpin ? 4 : 2) : (vpin ? 3 : 1);
+    const int src_ch = (chan == 1) ? 1 : ((chan == 0) == mp ? 2 : 0);
+    P.exch = ex ? 1 : 0;
+    P.flags = (smn ? 1 : 0) | (sm ? 2 : 0) | (sn ? 4 : 0);
+    P.sgn_d = sm != sn ? (R)-1 : (R)1;
+    const int64_t K1 = (int64_t)Ns * NO, K2 = K1 * Nn;  // sizes of q1, q2, q3 = K2 Nn
+    P.base = q0 + src_ch * (K1 + 2 * K2 + K2 * Nn) + (kernel == 1 ? 0 : K1 + (kernel - 2) * K2);
+    const auto p1 = find(w, M, oO, NO);
+    if (p1.lo < p1.hi) P.flags |= 8;
+    auto p2 = p1, p3 = p1;  // a fermionic argument beyond its mesh: one corner of weight 1
+    p2.lo = p2.hi = p3.lo = p3.hi = 0;
+    p2.wl = p3.wl = 1;
+    p2.wu = p3.wu = 0;
+    if (vin || vpin) p2 = find(vin ? v : vp, M, on, Nn);
+    if (kernel == 4) p3 = find(vp, M, on, Nn);
+    int n = 0;
+    const int n3 = p3.lo < p3.hi ? 2 : 1, n2 = p2.lo < p2.hi ? 2 : 1;
+#pragma unroll 1
+    for (int k = 0; k < n2 * n3; ++k) {
+        const bool u2 = n2 == 2 ? (k & 1) : false, u3 = n2 == 2 ? (k >> 1) : k;
+        const auto w2 = u2 ? p2.wu : p2.wl, w3 = u3 ? p3.wu : p3.wl;
+        const int o = Ns * NO * ((u2 ? p2.hi : p2.lo) + Nn * (u3 ? p3.hi : p3.lo));
+        P.w[n] = (R)(p1.wl * w2 * w3);
+        P.off[n++] = o + Ns * p1.lo;
+        if (p1.lo < p1.hi) {
+            P.w[n] = (R)(p1.wu * w2 * w3);
+            P.off[n++] = o + Ns * p1.hi;
+        }
+    }
+    P.nc = n;
+    return kernel;
+}
+
+// exp(x) and exp(x) - 1 for x <= 0, within an ulp of each.  x = k ln 2 + r with |r| <= ln(2)/2, the
+// Taylor sum of e^r - 1 to r^13 (the rest is below 1.2e-17 |r|) serves both: e^x - 1 = 2^k (e^r - 1) +
+// (2^k - 1), whose last bracket is exact.  23 FP64 operations instead of two library calls; largest error
+// seen on 2e7 arguments in (-700, 0): exp 0.86 ulp, exp - 1 0.90 ulp.
+static __device__ __noinline__ double exp_far(double x) { return exp(x); }
+__device__ __forceinline__ void exp_and_m1(double x, double& ex, double& em1) {
+    const double big = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer in the low bits
+    const double t = fma(x, 1.4426950408889634074, big);
+    const int k = __double2loint(t);
+    const double kd = t - big;
+    const double ln2l = 2.3190468138462996e-17;  // ln 2 - double(ln 2)
+    const double r0 = fma(kd, -0.69314718055994530942, x);
+    const double r = fma(kd, -ln2l, r0);
+    const double rl = fma(kd, -ln2l, r0 - r);  // what r lost in rounding
+    double q = 1.0 / 6227020800.0;
+    q = fma(q, r, 1.0 / 479001600.0);
+    q = fma(q, r, 1.0 / 39916800.0);
+    q = fma(q, r, 1.0 / 3628800.0);
+    q = fma(q, r, 1.0 / 362880.0);
+    q = fma(q, r, 1.0 / 40320.0);
+    q = fma(q, r, 1.0 / 5040.0);
+    q = fma(q, r, 1.0 / 720.0);
+    q = fma(q, r, 1.0 / 120.0);
+    q = fma(q, r, 1.0 / 24.0);
+    q = fma(q, r, 1.0 / 6.0);
+    q = fma(q, r, 0.5);
+    const double p = r + fma(r * r, q, rl);
+    const double s = __hiloint2double((k + 1023) << 20, 0);
+    ex = fma(s, p, s);
+    em1 = fma(s, p, s - 1.0);
+    // 2^k leaves the normal range (x < -700, x = -inf): e^x - 1 is -1 there
+    if (!(__double2hiint(x) >= 0) && (__double2hiint(x) & 0x7fffffff) >= 0x4085e000 && !is_nan(x)) {
+        ex = exp_far(x);
+        em1 = -1.0;
+    }
+}
+
+// What depends on one propagator frequency: G(w) and, for the Katanin bubble, K(w) = S(w) + G(w)^2 dΣ(w).
+// The bubbles are (K(w1) G(w2) + K(w2) G(w1)) / 2π and -G(w1) G(w2) / 2π (bubbles.jl:64-96).
+template <typename R>
+struct PropTerm {
+    R K, G;
+};
+
+// constants of the regulator exp(-w²/Λ²)
+struct PropConst {
+    double L2, iL2, twoL3;  // Λ², 1/Λ², 2/Λ³
+};
+
+// FP64: with E = 1 - exp(-w²/Λ²), G0 = E/w, G = E/(w + E Σ) and G/G0 = w/(w + E Σ) share one
+// reciprocal; Σ and dΣ share one interval search.  About 50 FP64 operations for a frequency; prop_half's
+// chain of library calls and divisions, both halves of which evaluate both frequencies, takes over ten
+// times as many for the two.  The FP64 pipe (two operations per clock and SM) bounds the FP64 passes: with
+// this, integer comparisons, one argument formula for all lanes and the compacted plans, square L = 3
+// FP64 right-hand sides took 65 instead of 193 ms (50/15/10, noise) and 4.0 instead of 18.8 ms (11/4/3),
+// kagome L = 3 U(1)-DM 29 instead of 45 ms, pyrochlore L = 6 92 instead of 105 ms.
+__device__ __forceinline__ PropTerm<double> prop_term(bool kat, const MeshD& M, const double* __restrict__ Sig,
+                                                      const double* __restrict__ dSig, const PropConst& c, double w) {
+    if (!(fabs(w) > 1e-8)) return PropTerm<double>{0.0, 0.0};
+    const int Nsig = M.Nsig;
+    const double aw = fabs(w);
+    double s, ds = 0.0;
+    if (!less_nonneg(M.at(M.sig(), Nsig - 1), aw)) {  // get_Σ (Action.jl:8-26)
+        const Param<double> p = get_param(aw, M.x, M.inv, Nsig);
+        const bool neg = __double2hiint(w) < 0;
+        s = p.wl * ldg(Sig + p.lo) + p.wu * ldg(Sig + p.hi);
+        s = neg ? -s : s;
+        if (kat) {
+            ds = p.wl * ldg(dSig + p.lo) + p.wu * ldg(dSig + p.hi);
+            ds = neg ? -ds : ds;
+        }
+    } else {
+        const double q = M.at(M.sig(), Nsig - 1) / w;
+        s = q * ldg(Sig + Nsig - 1);
+        if (kat) ds = q * ldg(dSig + Nsig - 1);
+    }
+    // w²/Λ² from the rounded reciprocal and one Newton correction of the quotient (Markstein 1990)
+    const double w2 = w * w;
+    double x = w2 * c.iL2;
+    x = fma(fma(-x, c.L2, w2), c.iL2, x);
+    if ((__double2hiint(c.iL2) & 0x7ff00000) >= 0x7fe00000) x = w2 / c.L2;  // Λ² at or near zero
+    double ex, em1;
+    exp_and_m1(-x, ex, em1);
+    // a Σ of the other sign than w is left out (G_full)
+    const double t = ((__double2hiint(w) ^ __double2hiint(s)) >= 0 && !is_nan(s)) ? s : 0.0;
+    const double inv = __drcp_rn(fma(-em1, t, w));
+    PropTerm<double> o;
+    o.G = -em1 * inv;
+    o.K = 0.0;
+    if (kat) {
+        const double r = w * inv;
+        o.K = fma(o.G * o.G, ds, r * r * ex * (c.twoL3 * w));
+    }
+    return o;
+}
+
+// FP32, float-float frequency: the operations of prop_half_ff's halves, each frequency once
+__device__ __forceinline__ PropTerm<float> prop_term(bool kat, const MeshFF& M, const float* __restrict__ Sig,
+                                                     const float* __restrict__ dSig, float L, FF a) {
+    PropTerm<float> o;
+    o.K = 0.f;
+    if (kat) {  // S(a) + G(a)^2 dΣ(a)
+        float ds = 0.f;
+        const float sa = get_sigma_ff(M, M.Nsig, Sig, a, dSig, &ds);
+        const float g1 = G_full_s(sa, L, a.h);
+        const float g0 = G_bare(L, a.h);
+        const float r = g1 / g0;
+        const float s1 = fabsf(a.h) > 1e-8f ? r * r * expf(-(a.h * a.h) / (L * L)) * 2.f * a.h / (L * L * L) : 0.f;
+        o.G = g1;
+        o.K = s1 + g1 * g1 * ds;
+    } else {
+        o.G = G_full_s(get_sigma_ff(M, M.Nsig, Sig, a), L, a.h);
+    }
+    return o;
+}
+__device__ __forceinline__ double prop_combine(bool kat, const PropTerm<double>* t) {
+    const double i2pi = 0.15915494309189533577;
+    return kat ? fma(t[0].K, t[1].G, t[1].K * t[0].G) * i2pi : -(t[0].G * t[1].G) * i2pi;
+}
+__device__ __forceinline__ float prop_combine(bool kat, const PropTerm<float>* t) {
+    if (!kat) return -(t[0].G * t[1].G) / two_pi<float>();
+    const float h0 = t[0].K * t[1].G / two_pi<float>();
+    const float h1 = t[1].K * t[0].G / two_pi<float>();
+    return h0 + h1;
+}
+
+// Plan arguments (flow_su2_s.jl:21-28, flow_su2_t.jl:21-43, flow_su2_u.jl:21-28) as a table: the
+// argument k of buffer (slot, channel) of bubble X is (a W + b v) + c F or half of that, with a, b, c in
+// {0, 1, -1} and F the first (slots 0, 2) or second (slots 1, 3) fermionic frequency of the task; the
+// sums run in the reference's order.  Seven bits per argument: two for each coefficient (1: +, 2: -), one
+// for the half.  One expression for every lane of a warp instead of one branch per buffer, whose
+// arithmetic the lanes of the other buffers waited for.
+constexpr unsigned arg_code(int a, int b, int c, int half) {
+    return (unsigned)((a < 0 ? 2 : a) | (b < 0 ? 2 : b) << 2 | (c < 0 ? 2 : c) << 4 | half << 6);
+}
+constexpr unsigned arg_codes(unsigned x, unsigned y, unsigned z) { return x | y << 7 | z << 14; }
+constexpr unsigned kW = arg_code(1, 0, 0, 0), kV = arg_code(0, 1, 0, 0), kF = arg_code(0, 0, 1, 0);
+constexpr unsigned kVmF = arg_code(0, 1, -1, 0), kVpF = arg_code(0, 1, 1, 0), kFmV = arg_code(0, -1, 1, 0);
+constexpr unsigned hc(int a, int b, int c) { return arg_code(a, b, c, 1); }
+static __device__ const unsigned kArgCodes[3][4][3] = {
+    {{arg_codes(kW, kF, arg_code(0, -1, 0, 0)), arg_codes(kVmF, hc(1, 1, 1), hc(1, -1, -1)), arg_codes(kVpF, hc(1, -1, 1), hc(1, 1, -1))},
+     {arg_codes(kW, kV, kF), arg_codes(arg_code(0, -1, -1, 0), hc(1, 1, -1), hc(1, -1, 1)), arg_codes(kVmF, hc(1, 1, 1), hc(1, -1, -1))}},
+    {{arg_codes(kVpF, hc(-1, -1, 1), hc(-1, 1, -1)), arg_codes(kW, kF, kV), arg_codes(kFmV, hc(-1, 1, 1), hc(1, 1, 1))},
+     {arg_codes(kVpF, hc(-1, 1, -1), hc(-1, -1, 1)), arg_codes(kW, kV, kF), arg_codes(kVmF, hc(-1, 1, 1), hc(1, 1, 1))},
+     {arg_codes(kVpF, hc(1, 1, -1), hc(-1, 1, -1)), arg_codes(kFmV, hc(1, 1, 1), hc(-1, 1, 1)), arg_codes(kW, kV, kF)},
+     {arg_codes(kVpF, hc(1, -1, 1), hc(-1, -1, 1)), arg_codes(kVmF, hc(1, 1, 1), hc(-1, 1, 1)), arg_codes(kW, kF, kV)}},
+    {{arg_codes(kVpF, hc(1, -1, 1), hc(-1, -1, 1)), arg_codes(kVmF, hc(1, 1, 1), hc(-1, 1, 1)), arg_codes(kW, kF, kV)},
+     {arg_codes(kVpF, hc(1, 1, -1), hc(-1, 1, -1)), arg_codes(kFmV, hc(1, 1, 1), hc(-1, 1, 1)), arg_codes(kW, kV, kF)}}};
+
+// 0, x or -x
+__device__ __forceinline__ double arg_term(unsigned s, double x) {
+    return s == 0 ? 0.0 : (s == 1 ? x : -x);
+}
+__device__ __forceinline__ FF arg_term(unsigned s, FF x) {
+    return s == 0 ? FF{0.f, 0.f} : (s == 1 ? x : -x);
+}
+__device__ __forceinline__ double arg_half(unsigned h, double x) { return (h ? 0.5 : 1.0) * x; }
+__device__ __forceinline__ FF arg_half(unsigned h, FF x) { return FF{h ? 0.5f : 1.f, 0.f} * x; }
+template <typename S>
+__device__ __forceinline__ S plan_arg(unsigned code, S W, S v, S F) {
+    return arg_half((code >> 6) & 1, (arg_term(code & 3, W) + arg_term((code >> 2) & 3, v)) + arg_term((code >> 4) & 3, F));
+}
+// the propagator frequencies of bubble X: v ± W/2 (bubbles.jl:99-221)
+template <typename S>
+__device__ __forceinline__ S prop_freq(int X, int item, S v, S hW) {
+    if (X == 0 && item == 1) return hW + (-v);
+    return v + ((X == 2) == (item == 1) ? hW : -hW);
 }
 
 // prop_half with float-float frequencies (bubbles.jl:64-96)

@@ -50,9 +50,10 @@ constexpr int kWarps = 4;
 template <typename R, int C>
 struct NodeScratch {
     double x;      // the node (integration variable v)
-    R p_half[2];
+    PropTerm<R> prop[2];
+    R p;           // the bubble propagator
     R loc[2 * C];  // t channel: local vertices v3[C], v4[C] at site 1
-    Plan<R> plan[4][3];
+    NodePlan<R> plan[4][3];
 };
 
 // nodes per team batch: 4 per warp in total, 2 for SU(2) when each lane holds more than four sites
@@ -123,93 +124,34 @@ __device__ __forceinline__ void u1dm_t(const R* v1, const R* v2, const R* v3, co
            (R)2 * v3[2] * v2[1] + v3[1] * v2[5];
 }
 
-// per-node argument triple (w, v, v') of buffer (slot, ch) for channel X
-// (flow_su2_s.jl:21-28, flow_su2_t.jl:21-43, flow_su2_u.jl:21-28)
-template <typename R>
-__device__ __forceinline__ void slot_arg(int X, int slot, int ch, R v, R W, R V, R VP, R& a0, R& a1, R& a2) {
-    const R h = (R)0.5;
-    if (X == 0) {
-        const R s = W, vs = V, vsp = VP;
-        if (slot == 0) {
-            if (ch == 0) { a0 = s; a1 = vs; a2 = -v; }
-            else if (ch == 1) { a0 = v - vs; a1 = h * (s + v + vs); a2 = h * (s - v - vs); }
-            else { a0 = v + vs; a1 = h * (s - v + vs); a2 = h * (s + v - vs); }
-        } else {
-            if (ch == 0) { a0 = s; a1 = v; a2 = vsp; }
-            else if (ch == 1) { a0 = -v - vsp; a1 = h * (s + v - vsp); a2 = h * (s - v + vsp); }
-            else { a0 = v - vsp; a1 = h * (s + v + vsp); a2 = h * (s - v - vsp); }
-        }
-    } else if (X == 1) {
-        const R t = W, vt = V, vtp = VP;
-        switch (slot) {
-            case 0:
-                if (ch == 0) { a0 = v + vt; a1 = h * (-t - v + vt); a2 = h * (-t + v - vt); }
-                else if (ch == 1) { a0 = t; a1 = vt; a2 = v; }
-                else { a0 = -v + vt; a1 = h * (-t + v + vt); a2 = h * (t + v + vt); }
-                break;
-            case 1:
-                if (ch == 0) { a0 = v + vtp; a1 = h * (-t + v - vtp); a2 = h * (-t - v + vtp); }
-                else if (ch == 1) { a0 = t; a1 = v; a2 = vtp; }
-                else { a0 = v - vtp; a1 = h * (-t + v + vtp); a2 = h * (t + v + vtp); }
-                break;
-            case 2:
-                if (ch == 0) { a0 = v + vt; a1 = h * (t + v - vt); a2 = h * (-t + v - vt); }
-                else if (ch == 1) { a0 = -v + vt; a1 = h * (t + v + vt); a2 = h * (-t + v + vt); }
-                else { a0 = t; a1 = v; a2 = vt; }
-                break;
-            default:
-                if (ch == 0) { a0 = v + vtp; a1 = h * (t - v + vtp); a2 = h * (-t - v + vtp); }
-                else if (ch == 1) { a0 = v - vtp; a1 = h * (t + v + vtp); a2 = h * (-t + v + vtp); }
-                else { a0 = t; a1 = vtp; a2 = v; }
-                break;
-        }
-    } else {
-        const R u = W, vu = V, vup = VP;
-        if (slot == 0) {
-            if (ch == 0) { a0 = v + vu; a1 = h * (u - v + vu); a2 = h * (-u - v + vu); }
-            else if (ch == 1) { a0 = v - vu; a1 = h * (u + v + vu); a2 = h * (-u + v + vu); }
-            else { a0 = u; a1 = vu; a2 = v; }
-        } else {
-            if (ch == 0) { a0 = v + vup; a1 = h * (u + v - vup); a2 = h * (-u + v - vup); }
-            else if (ch == 1) { a0 = -v + vup; a1 = h * (u + v + vup); a2 = h * (-u + v + vup); }
-            else { a0 = u; a1 = v; a2 = vup; }
-        }
-    }
-}
-
 // vertex component c of one slot at one site (single value), for the t-channel local vertices
 template <typename R, int C>
 __device__ __forceinline__ R gather_one(const PassArgs<R>& A, const NodeScratch<R, C>& ns, int slot, int c, int i,
                                         int exch_i) {
     const R* __restrict__ src = A.src[slot];
-    if constexpr (sizeof(R) == 4 && C == 2) {
-        // FP32 copies of SU(2) actions hold (spin, density) pairs
-        const float* __restrict__ s2 = src + c;
-        R val = ldg(s2 + 2 * (A.L.pbare() + i));
-#pragma unroll
-        for (int ch = 0; ch < 3; ++ch) {
-            const Plan<R>& P = ns.plan[slot][ch];
-            if (P.kernel) {
-                const float* q = s2 + 2 * A.L.pq(P.src_ch, P.kernel - 1);
-                const int s = P.exch ? exch_i : i;
-                R acc = P.w[0] * ldg(q + 2 * (P.off[0] + s));
-                for (int k = 1; k < corners_of(P.kernel); ++k) acc += P.w[k] * ldg(q + 2 * (P.off[k] + s));
-                val += (c == 1 ? P.sgn_d : (R)1) * acc;
+    constexpr int CS = sizeof(R) == 4 && C == 2 ? 2 : 1;  // FP32 copies of SU(2) actions hold (spin, density) pairs
+    R val = CS == 2 ? ldg(src + c + 2 * (A.L.pbare() + i)) : ldg(src + A.L.bare(c) + i);
+#pragma unroll 1
+    for (int ch = 0; ch < 3; ++ch) {
+        const NodePlan<R>& P = ns.plan[slot][ch];
+        const int nc = P.nc;
+        if (!nc) continue;
+        R sgn;
+        const int cs = comp_read(P, C, c, sgn);
+        const R* q = CS == 2 ? src + c + 2 * P.base : src + P.base + cs * A.L.comp;
+        const int st = P.exch ? exch_i : i;
+        R acc = P.w[0] * ldg(q + CS * (P.off[0] + st));
+        int k = 1;
+        if constexpr (sizeof(R) == 4 && C == 6) {
+            // the second product of a bosonic pair is rounded first: the FP32 results stay those of the
+            // uncompacted plan, in which the compiler chose this order (either is as exact)
+            if (P.flags & 8) {
+                acc = fmaf(P.w[0], ldg(q + P.off[0] + st), __fmul_rn(P.w[1], ldg(q + P.off[1] + st)));
+                k = 2;
             }
         }
-        return val;
-    }
-    R val = ldg(src + A.L.bare(c) + i);
-#pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
-        const Plan<R>& P = ns.plan[slot][ch];
-        if (P.kernel) {
-            R sgn;
-            const int cs = comp_read(P, C, c, sgn);
-            const R* q = src + A.L.qbase(cs, P.src_ch, P.kernel - 1);
-            R acc = plan_read(P, q, P.exch ? exch_i : i);
-            val += sgn * acc;
-        }
+        for (; k < nc; ++k) acc += P.w[k] * ldg(q + CS * (P.off[k] + st));
+        val += sgn * acc;
     }
     return val;
 }
@@ -237,12 +179,11 @@ __device__ __forceinline__ void gather_slot(const PassArgs<R>& A, const NodeScra
     for (int k = 0; k < SPL; ++k)
 #pragma unroll
         for (int c = 0; c < C; ++c) v[c][k] = ldg(src + A.L.bare(c) + si[k]);
-#pragma unroll
+#pragma unroll 1
     for (int ch = 0; ch < 3; ++ch) {
-        const Plan<R>& P = ns.plan[slot][ch];
-        const int kern = P.kernel;
-        if (!kern) continue;
-        const int nc = corners_of(kern);
+        const NodePlan<R>& P = ns.plan[slot][ch];
+        const int nc = P.nc;
+        if (!nc) continue;
         int st[SPL];
 #pragma unroll
         for (int k = 0; k < SPL; ++k) st[k] = P.exch ? site_ex[k] : si[k];
@@ -251,7 +192,7 @@ __device__ __forceinline__ void gather_slot(const PassArgs<R>& A, const NodeScra
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             const int cs = comp_read(P, C, c, sg[c]);
-            q0[c] = src + A.L.qbase(cs, P.src_ch, kern - 1);
+            q0[c] = src + P.base + cs * A.L.comp;
         }
         R a[C][SPL];
 #pragma unroll
@@ -318,12 +259,25 @@ __device__ __forceinline__ TaskInfo task_of(const PassArgs<R>& A, int sub, int j
     return TaskInfo{A.chan_of_y[y], t.x, t.y, t.z, t.w};
 }
 
+// The plan of a mixed-path argument near a buffer switch: the FP64 path's rounding decides the side.
+// Not inlined (and given values, not the kernel's arguments, whose address would copy them to local
+// memory): few lanes take it, and the kernels' code has to fit the instruction caches.
+static __device__ __noinline__ int plan_fp64(NodePlan<float>& P, const double* mesh, int Nsig, int NO, int Nn, int Ns,
+                                             int64_t q0, int X, int w1, int wf, int ch, unsigned code,
+                                             double x) {
+    const MeshD M = mesh_view_d(mesh, Nsig, NO, Nn);
+    const double W = M.at(X == 1 ? M.Ot() : M.Os(), w1);
+    const double F = wf >= 0 ? M.at(X == 1 ? M.nt() : M.ns(), wf) : INFINITY;
+    return build_plan(P, ch, plan_arg(code, W, x, F), plan_arg(code >> 7, W, x, F), plan_arg(code >> 14, W, x, F), M, Ns,
+                      q0);
+}
+
 template <typename R, int T, int SPL, int C>
 struct Team {
     const PassArgs<R>& A;
     // node setup: FP64 on the FP64 path, float-float on the mixed path
     using SetupT = typename std::conditional<sizeof(R) == 4, FF, double>::type;
-    using SetupMesh = typename std::conditional<sizeof(R) == 4, MeshFF, MeshG<double>>::type;
+    using SetupMesh = typename std::conditional<sizeof(R) == 4, MeshFF, MeshD>::type;
     const SetupMesh& M;
     TeamScratch<R, T, C, SPL>& ts;
     R* tmp;                 // t channel: [2 C][Ns] slot values of the current node
@@ -332,6 +286,11 @@ struct Team {
     int tl;                 // lane in team
     int site_ex[SPL];       // exchange[site] of this lane's sites
     unsigned long long nodes, alg;
+
+    // offset of the first kernel of the s channel in a vertex source
+    __device__ __forceinline__ int64_t q0() const {
+        return sizeof(R) == 4 && C == 2 ? A.L.pbare() + A.L.Ns : A.L.qbase(0, 0, 0);
+    }
 
     // Evaluate the integrand of channel X at the up to NB nodes ts.node[0..count).x of one task and
     // hand each node's values to sink(j, g) in node order, g[c][k] = Γ_c(site tl + k T; x_j)
@@ -342,8 +301,8 @@ struct Team {
         const int X = ti.X;
         const int Ns = A.L.Ns;
         const int nslots = (X == 1) ? 4 : 2;
-        const int nprop = A.prop_kind == PROP_KAT ? 2 : 1;
-        const int nitems = nprop + 3 * nslots;
+        const bool kat = A.prop_kind == PROP_KAT;
+        const int nitems = 2 + 3 * nslots;
         nodes += count;
         // teams of one warp may hold different channels and batch lengths: every lane runs
         // the same sequence of warp syncs, bounded by the warp's longest batch
@@ -351,48 +310,53 @@ struct Team {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
         // phase A: scalar work of all nodes of the batch, split over the team's lanes
+        unsigned corners = 0;  // corners of this lane's plans times the sites that read them
+#pragma unroll 1
         for (int it = tl; it < count * nitems; it += T) {
             const int j = it / nitems, item = it - j * nitems;
             NodeScratch<R, C>& ns = ts.node[j];
             const double xj = ns.x;
             const SetupT v = SetupT(xj);
-            if (item < nprop) {
+            if (item < 2) {
                 if constexpr (sizeof(R) == 4)
-                    ns.p_half[item] = prop_half_ff(A.prop_kind, item, X, M, A.L.Nsig, A.prop_a, A.prop_da,
-                                                   (float)A.Lam, v, W);
+                    ns.prop[item] = prop_term(kat, M, A.prop_a, A.prop_da, (float)A.Lam,
+                                              prop_freq(X, item, v, FF{0.5f, 0.f} * W));
                 else
-                    ns.p_half[item] = prop_half<double>(A.prop_kind, item, X, M, A.L.Nsig, A.prop_a64, A.prop_da64,
-                                                        A.Lam, v, W);
-            } else {
-                const int k = item - nprop;
-                const int slot = k / 3, ch = k - 3 * slot;
-                Plan<R>& P = ns.plan[slot][ch];
-                if (A.mask[X][slot] & (1 << ch)) {
-                    SetupT a0, a1, a2;
-                    slot_arg<SetupT>(X, slot, ch, v, W, V, VP, a0, a1, a2);
-                    if constexpr (sizeof(R) == 4) {
-                        const float scale = fabsf(v.h) + fabsf(W.h) + (isinf(V.h) ? 0.f : fabsf(V.h)) +
-                                            (isinf(VP.h) ? 0.f : fabsf(VP.h));
-                        if (ff_near_switch(a0, scale, M, A.L.NO, A.L.Nn) || ff_near_switch(a1, scale, M, A.L.NO, A.L.Nn) ||
-                            ff_near_switch(a2, scale, M, A.L.NO, A.L.Nn)) {
-                            // the FP64 path's rounding decides the side of a buffer switch
-                            const MeshG<double> M64 = mesh_view(A.mesh, A.L.Nsig, A.L.NO, A.L.Nn);
-                            double W64, V64, VP64, b0, b1, b2;
-                            task_freqs(A, M64, ti, W64, V64, VP64);
-                            slot_arg<double>(X, slot, ch, xj, W64, V64, VP64, b0, b1, b2);
-                            make_plan<R>(P, ch, b0, b1, b2, M64, Ns, A.L.NO, A.L.Nn);
-                        } else {
-                            make_plan_ff(P, ch, a0, a1, a2, M, Ns, A.L.NO, A.L.Nn);
-                        }
-                    } else {
-                        make_plan<R>(P, ch, a0, a1, a2, M, Ns, A.L.NO, A.L.Nn);
-                    }
-                } else {
-                    P.kernel = 0;
-                }
+                    ns.prop[item] = prop_term(kat, M, A.prop_a64, A.prop_da64, A.pc, prop_freq(X, item, v, 0.5 * W));
+                continue;
             }
+            const int k = item - 2;
+            const int slot = k / 3, ch = k - 3 * slot;
+            NodePlan<R>& P = ns.plan[slot][ch];
+            if (!(A.mask[X][slot] & (1 << ch))) {
+                P.nc = 0;
+                continue;
+            }
+            const unsigned code = __ldg(&kArgCodes[X][slot][ch]);
+            const SetupT F = (slot & 1) ? VP : V;
+            const SetupT a0 = plan_arg(code, W, v, F), a1 = plan_arg(code >> 7, W, v, F),
+                         a2 = plan_arg(code >> 14, W, v, F);
+            int kernel;
+            if constexpr (sizeof(R) == 4) {
+                const float scale = fabsf(v.h) + fabsf(W.h) + (isinf(V.h) ? 0.f : fabsf(V.h)) +
+                                    (isinf(VP.h) ? 0.f : fabsf(VP.h));
+                if (ff_near_switch(a0, scale, M, A.L.NO, A.L.Nn) || ff_near_switch(a1, scale, M, A.L.NO, A.L.Nn) ||
+                    ff_near_switch(a2, scale, M, A.L.NO, A.L.Nn))
+                    kernel = plan_fp64(P, A.mesh, A.L.Nsig, A.L.NO, A.L.Nn, Ns, q0(), X, ti.w1, (slot & 1) ? ti.w3 : ti.w2,
+                                       ch, code, xj);
+                else
+                    kernel = build_plan(P, ch, a0, a1, a2, M, Ns, q0());
+            } else {
+                kernel = build_plan(P, ch, a0, a1, a2, M, Ns, q0());
+            }
+            corners += corners_of(kernel) * (slot < 2 ? Ns : 1);
+        }
+        if (A.node_counter) {
+            alg += (unsigned long long)corners * C;
+            if (tl == 0) alg += (unsigned long long)count * C * (3ull * Ns + (X == 1 ? 2ull * row_off[Ns] : 0ull));
         }
         __syncwarp();
+        if (tl < count) ts.node[tl].p = prop_combine(kat, ts.node[tl].prop);
         if (X == 1) {
             // local vertices at site 1 (flow_su2_t.jl:46-48, flow_u1_dm_t.jl:44-46)
             const int e0 = ldg(A.exch);
@@ -402,16 +366,6 @@ struct Team {
             }
         }
         __syncwarp();
-        if (A.node_counter && tl == 0) {
-            for (int j = 0; j < count; ++j) {
-                unsigned long long cs = 0, c1 = 0;
-                for (int s = 0; s < nslots; ++s)
-                    for (int ch = 0; ch < 3; ++ch) (s < 2 ? cs : c1) += corners_of(ts.node[j].plan[s][ch].kernel);
-                unsigned long long v = cs * Ns + c1 + 3ull * Ns;
-                if (X == 1) v += 2ull * row_off[Ns];
-                alg += v * C;
-            }
-        }
         if constexpr (C == 2) {
             // every team of the warp passes the same two warp barriers, whatever its channel
             eval_su2_nodes(X, count, sink);
@@ -427,7 +381,7 @@ struct Team {
             R p = (R)0;
             R v1[C][SPL], v2[C][SPL];
             if (act) {
-                p = (nprop == 2) ? ns.p_half[0] + ns.p_half[1] : ns.p_half[0];
+                p = ns.p;
                 gather_slot<R, T, SPL, C>(A, ns, 0, tl, site_ex, v1);
                 gather_slot<R, T, SPL, C>(A, ns, 1, tl, site_ex, v2);
             }
@@ -461,13 +415,12 @@ struct Team {
                 v[0][k] = b.x;
                 v[1][k] = b.y;
             }
-#pragma unroll
+#pragma unroll 1
             for (int ch = 0; ch < 3; ++ch) {
-                const Plan<R>& P = ns.plan[slot][ch];
-                const int kern = P.kernel;
-                if (!kern) continue;
-                const int nc = corners_of(kern);
-                const float2* q = src2 + A.L.pq(P.src_ch, kern - 1);
+                const NodePlan<R>& P = ns.plan[slot][ch];
+                const int nc = P.nc;
+                if (!nc) continue;
+                const float2* q = src2 + P.base;
                 const R sgn_d = P.sgn_d;
                 const int ex = P.exch;
                 int st[SPL];
@@ -504,14 +457,13 @@ struct Team {
             v[0][k] = ldg(src + A.L.bare(0) + si[k]);
             v[1][k] = ldg(src + A.L.bare(1) + si[k]);
         }
-#pragma unroll
+#pragma unroll 1
         for (int ch = 0; ch < 3; ++ch) {
-            const Plan<R>& P = ns.plan[slot][ch];
-            const int kern = P.kernel;
-            if (!kern) continue;
-            const int nc = corners_of(kern);
-            const R* q0 = src + A.L.qbase(0, P.src_ch, kern - 1);
-            const R* q1 = src + A.L.qbase(1, P.src_ch, kern - 1);
+            const NodePlan<R>& P = ns.plan[slot][ch];
+            const int nc = P.nc;
+            if (!nc) continue;
+            const R* q0 = src + P.base;
+            const R* q1 = q0 + A.L.comp;
             const R sgn_d = P.sgn_d;
             const int ex = P.exch;
             int st[SPL];
@@ -557,7 +509,7 @@ struct Team {
         const R two = (X == 0) ? (R)-2 : (R)2;
         for (int j = 0; j < count; ++j) {
             const NodeScratch<R, C>& ns = ts.node[j];
-            const R p = ns.p_half[0] + (A.prop_kind == PROP_KAT ? ns.p_half[1] : (R)0);
+            const R p = ns.p;
             R v1[2][SPL], v2[2][SPL];
             gather_su2(ns, 0, v1);
             gather_su2(ns, 1, v2);
@@ -670,7 +622,7 @@ struct Team {
         for (int jj = 0; jj < NB; ++jj) {
             if (jj >= count) continue;
             const NodeScratch<R, C>& ns = ts.node[jj];
-            const R p = ns.p_half[0] + (A.prop_kind == PROP_KAT ? ns.p_half[1] : (R)0);
+            const R p = ns.p;
             const R coef = -p * (R)-2 * twoS;
             R g[2][SPL];
 #pragma unroll
@@ -684,6 +636,21 @@ struct Team {
                 }
             }
             sink(jj, g);
+        }
+    }
+
+    // add this warp's evaluations and algorithmic values to the context's counters
+    __device__ __forceinline__ void count_nodes() {
+        if (!A.node_counter) return;
+        unsigned long long n = tl == 0 ? nodes : 0, a = alg;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            n += __shfl_xor_sync(kFull, n, o);
+            a += __shfl_xor_sync(kFull, a, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(A.node_counter, n);
+            atomicAdd(A.node_counter + 1, a);
         }
     }
 
@@ -794,7 +761,10 @@ struct LevelCut {
 // team takes for 32 nodes one after another (square L = 3 FP64: 93, 166, 308 and 570 us for chunks of 4,
 // 8, 16 and 32 nodes; kagome L = 8 FP64: 10 ms for every level).  Chunks are therefore halved, down to one
 // batch of nodes, while the level still has fewer chunks than `teams`, about twice the teams that the GPU
-// holds at once; larger levels keep the coarse cut, whose partial sums cost least.
+// holds at once; larger levels keep the coarse cut, whose partial sums cost least.  Right-hand sides and
+// steps, coarse cut only against this rule: square L = 3 11/4/3 FP64 40.1 -> 18.8 ms and 50/15/10 mixed
+// 34.1 -> 22.1 ms, kagome L = 8 U(1)-DM three loops mixed 482 -> 293 ms, honeycomb L = 5 two-loop step mixed
+// 222 -> 167 ms, pyrochlore L = 6 two loops mixed 377 -> 351 ms.
 __host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, int batch, int teams) {
     LevelCut k;
     const int per0 = n <= (long long)kChunk * kMaxChunks ? (int)(n < kChunk ? n : kChunk) : (int)(n / kMaxChunks);
@@ -829,7 +799,7 @@ __device__ __forceinline__ void enqueue(WaveSpace& Wsp, int par, int sub) {
 template <typename R>
 __device__ __forceinline__ auto setup_mesh(const PassArgs<R>& A, const unsigned char* smem) {
     if constexpr (sizeof(R) == 4) return mesh_view_ff(reinterpret_cast<const float*>(smem), A.L.Nsig, A.L.NO, A.L.Nn);
-    else return mesh_view(reinterpret_cast<const double*>(smem), A.L.Nsig, A.L.NO, A.L.Nn);
+    else return mesh_view_d(reinterpret_cast<const double*>(smem), A.L.Nsig, A.L.NO, A.L.Nn);
 }
 
 template <typename R>
@@ -844,10 +814,10 @@ __device__ __forceinline__ void task_freqs(const PassArgs<R>& A, const MeshFF& M
 }
 
 template <typename R>
-__device__ __forceinline__ void task_freqs(const PassArgs<R>& A, const MeshG<double>& M, const TaskInfo& ti, double& W,
+__device__ __forceinline__ void task_freqs(const PassArgs<R>& A, const MeshD& M, const TaskInfo& ti, double& W,
                                            double& V, double& VP) {
-    const double* Om = (ti.X == 1) ? M.Ot : M.Os;
-    const double* nu = (ti.X == 1) ? M.nt : M.ns;
+    const double* Om = M.x + (ti.X == 1 ? M.Ot() : M.Os());
+    const double* nu = M.x + (ti.X == 1 ? M.nt() : M.ns());
     const double inf = INFINITY;
     W = Om[ti.w1];
     V = (ti.kernel == 2 || ti.kernel == 4) ? nu[ti.w2] : inf;
@@ -1087,6 +1057,7 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
         if (valid) task_freqs(A, M, ti, W, V, VP);
         // all teams of the warp evaluate together (cnt = 0 for idle teams), NB nodes at a time
         R g[5][C][SPL];
+#pragma unroll 1
         for (int b = 0; b < 5; b += NB) {
             const int nb = max(0, min(NB, cnt - b));
             for (int j = tl; j < nb; j += T) tm.ts.node[j].x = x[b + j];
@@ -1181,10 +1152,7 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
             if (!done) enqueue(Wsp, 1, sub);
         }
     }
-    if (A.node_counter && tl == 0) {
-        atomicAdd(A.node_counter, tm.nodes);
-        atomicAdd(A.node_counter + 1, tm.alg);
-    }
+    tm.count_nodes();
 }
 
 // ---- wave k >= 1: evaluate queued chunks, one partial node sum per chunk ----
@@ -1259,6 +1227,7 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
                     if constexpr (sizeof(R) == 4) aab[c][k] += fabsf(gv[c][k]);
                 }
         };
+#pragma unroll 1
         for (int b = 0; b < K.per; b += NB) {
             const int nb = max(0, min(NB, cnt - b));
             if (tl < nb) {
@@ -1302,10 +1271,7 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
             }
         }
     }
-    if (A.node_counter && tl == 0) {
-        atomicAdd(A.node_counter, tm.nodes);
-        atomicAdd(A.node_counter + 1, tm.alg);
-    }
+    tm.count_nodes();
 }
 
 // ---- wave k >= 1: per subdomain, next Simpson sum, test, result or next level ----
@@ -1495,6 +1461,8 @@ struct PassLauncher {
         // blocks (three for FP64) still fits on an SM (228 KB less 1 KB per block; a row word is read
         // once per batch of nodes, so from L1 it costs little)
         PassArgs<R> a = a0;
+        const double L2 = a.Lam * a.Lam;
+        a.pc = PropConst{L2, 1.0 / L2, 2.0 / (a.Lam * a.Lam * a.Lam)};
         const int nm = a.L.Nsig + 2 * a.L.NO + 2 * a.L.Nn;
         const size_t staged = SmemLayout<R, T, C, SPL>(a.L.Ns, nm, a.rows_total, true).total;
         constexpr int fit_kb = 228 / (sizeof(R) == 4 ? eval_min_blocks<R, T, SPL, C>() : 3) - 1;

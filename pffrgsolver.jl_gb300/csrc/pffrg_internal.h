@@ -51,6 +51,7 @@ struct PassArgs {
     int nchan;            // channels launched (3, or 1 for the reduced s bubble)
     int chan_of_y[3];     // blockIdx.y -> channel
     double Lam, atol, rtol;
+    PropConst pc;         // from Lam, set at the launch
     int eval;
     double twoS;
     int reduced;          // reduced s bubble of the SDE (U(1)-DM keeps xx, zz, dd only)

@@ -83,45 +83,67 @@ struct TeamScratch {
 // reference's term order; the same combination serves the Katanin, left,
 // central, BSE and reduced kernels of a channel
 // ---------------------------------------------------------------------------
+// a0 b0 + a1 b1 + ...: the second product is rounded, the others enter by fused multiply-adds.  Written out
+// because a compiler that chooses which products to fuse chooses differently from one kernel to the next.
+template <typename R>
+__device__ __forceinline__ R terms_from(R acc) {
+    return acc;
+}
+template <typename R, typename... T>
+__device__ __forceinline__ R terms_from(R acc, R a, R b, T... rest) {
+    return terms_from(fma(a, b, acc), rest...);
+}
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+template <typename R, typename... T>
+__device__ __forceinline__ R terms(R a0, R b0, R a1, R b1, T... rest) {
+    return terms_from(fma(a0, b0, mul_rn(a1, b1)), rest...);
+}
 // s channel (flow_u1_dm_s.jl:53-58)
 template <typename R>
 __device__ __forceinline__ void u1dm_s(const R* a, const R* b, R* g) {
-    g[0] = a[2] * b[5] - a[2] * b[4] + a[0] * b[3] + a[3] * b[0] - a[0] * b[1] - a[5] * b[2] + a[4] * b[2] - a[1] * b[0];
-    g[1] = a[1] * b[3] + a[3] * b[1] - a[5] * b[4] - (R)2 * a[0] * b[0] - (R)2 * a[2] * b[2] - a[4] * b[5];
-    g[2] = a[3] * b[2] + a[2] * b[3] - a[4] * b[0] - a[0] * b[5] - a[1] * b[2] + a[0] * b[4] - a[2] * b[1] + a[5] * b[0];
-    g[3] = -a[5] * b[5] + (R)2 * a[0] * b[0] + a[3] * b[3] + (R)2 * a[2] * b[2] - a[4] * b[4] + a[1] * b[1];
-    g[4] = a[4] * b[3] + a[3] * b[4] - (R)2 * a[2] * b[0] + a[5] * b[1] + a[1] * b[5] + (R)2 * a[0] * b[2];
-    g[5] = a[4] * b[1] + a[3] * b[5] + a[1] * b[4] + (R)2 * a[2] * b[0] + a[5] * b[3] - (R)2 * a[0] * b[2];
+    g[0] = terms(a[2], b[5], -a[2], b[4], a[0], b[3], a[3], b[0], -a[0], b[1], -a[5], b[2], a[4], b[2],
+                 -a[1], b[0]);
+    const R m0 = mul_rn((R)2 * a[0], b[0]);
+    g[1] = terms_from(terms(a[1], b[3], a[3], b[1], -a[5], b[4]) - m0, -((R)2 * a[2]), b[2], -a[4], b[5]);
+    g[2] = terms(a[3], b[2], a[2], b[3], -a[4], b[0], -a[0], b[5], -a[1], b[2], a[0], b[4], -a[2], b[1],
+                 a[5], b[0]);
+    g[3] = terms_from(fma(-a[5], b[5], m0), a[3], b[3], (R)2 * a[2], b[2], -a[4], b[4], a[1], b[1]);
+    g[4] = terms(a[4], b[3], a[3], b[4], -((R)2 * a[2]), b[0], a[5], b[1], a[1], b[5], (R)2 * a[0], b[2]);
+    g[5] = terms(a[4], b[1], a[3], b[5], a[1], b[4], (R)2 * a[2], b[0], a[5], b[3], -((R)2 * a[0]), b[2]);
 }
 // u channel (flow_u1_dm_u.jl:52-57)
 template <typename R>
 __device__ __forceinline__ void u1dm_u(const R* a, const R* b, R* g) {
-    g[0] = -a[2] * b[5] - a[2] * b[4] + a[0] * b[3] + a[3] * b[0] + a[0] * b[1] + a[5] * b[2] + a[4] * b[2] + a[1] * b[0];
-    g[1] = a[1] * b[3] + a[3] * b[1] - a[5] * b[4] + (R)2 * a[0] * b[0] + (R)2 * a[2] * b[2] - a[4] * b[5];
-    g[2] = a[3] * b[2] + a[2] * b[3] - a[4] * b[0] + a[0] * b[5] + a[1] * b[2] + a[0] * b[4] + a[2] * b[1] - a[5] * b[0];
-    g[3] = -a[5] * b[5] + (R)2 * a[0] * b[0] + a[3] * b[3] + (R)2 * a[2] * b[2] - a[4] * b[4] + a[1] * b[1];
-    g[4] = a[4] * b[3] + a[3] * b[4] - (R)2 * a[2] * b[0] + a[5] * b[1] + a[1] * b[5] + (R)2 * a[0] * b[2];
-    g[5] = a[4] * b[1] + a[3] * b[5] + a[1] * b[4] - (R)2 * a[2] * b[0] + a[5] * b[3] + (R)2 * a[0] * b[2];
+    g[0] = terms(-a[2], b[5], -a[2], b[4], a[0], b[3], a[3], b[0], a[0], b[1], a[5], b[2], a[4], b[2],
+                 a[1], b[0]);
+    const R m0 = mul_rn((R)2 * a[0], b[0]);
+    g[1] = terms_from(terms(a[1], b[3], a[3], b[1], -a[5], b[4]) + m0, (R)2 * a[2], b[2], -a[4], b[5]);
+    g[2] = terms(a[3], b[2], a[2], b[3], -a[4], b[0], a[0], b[5], a[1], b[2], a[0], b[4], a[2], b[1],
+                 -a[5], b[0]);
+    g[3] = terms_from(fma(-a[5], b[5], m0), a[3], b[3], (R)2 * a[2], b[2], -a[4], b[4], a[1], b[1]);
+    g[4] = terms(a[4], b[3], a[3], b[4], -((R)2 * a[2]), b[0], a[5], b[1], a[1], b[5], (R)2 * a[0], b[2]);
+    g[5] = terms(a[4], b[1], a[3], b[5], a[1], b[4], -((R)2 * a[2]), b[0], a[5], b[3], (R)2 * a[0], b[2]);
 }
 // t channel, local part: v1, v2 non-local at site i, v3, v4 local at site 1 (flow_u1_dm_t.jl:68-84)
 template <typename R>
 __device__ __forceinline__ void u1dm_t(const R* v1, const R* v2, const R* v3, const R* v4, R* g) {
-    g[0] = v1[2] * v4[5] - v1[2] * v4[4] + v1[0] * v4[3] - v1[0] * v4[1] + v3[3] * v2[0] + v3[5] * v2[2] -
-           v3[4] * v2[2] - v3[1] * v2[0];
-    g[1] = v1[1] * v4[3] + (R)2 * v1[4] * v4[2] - v1[4] * v4[4] + v1[1] * v4[1] - (R)2 * v1[1] * v4[0] -
-           v1[4] * v4[5] - (R)2 * v3[2] * v2[5] - v3[5] * v2[5] + v3[3] * v2[1] - (R)2 * v3[0] * v2[1] +
-           v3[1] * v2[1] - v3[4] * v2[5];
-    g[2] = v1[2] * v4[3] - v1[0] * v4[5] + v1[0] * v4[4] - v1[2] * v4[1] - v3[5] * v2[0] + v3[3] * v2[2] +
-           v3[4] * v2[0] - v3[1] * v2[2];
-    g[3] = -v1[5] * v4[5] + (R)2 * v1[3] * v4[0] + v1[3] * v4[1] - v1[5] * v4[4] - (R)2 * v1[5] * v4[2] +
-           v1[3] * v4[3] + (R)2 * v3[2] * v2[4] + (R)2 * v3[0] * v2[3] + v3[1] * v2[3] - v3[5] * v2[4] +
-           v3[3] * v2[3] - v3[4] * v2[4];
-    g[4] = v1[4] * v4[1] + v1[4] * v4[3] + (R)2 * v1[4] * v4[0] + v1[1] * v4[4] + (R)2 * v1[1] * v4[2] +
-           v1[1] * v4[5] + v3[4] * v2[3] + (R)2 * v3[2] * v2[3] + v3[3] * v2[4] + v3[1] * v2[4] -
-           (R)2 * v3[0] * v2[4] + v3[5] * v2[3];
-    g[5] = -(R)2 * v1[3] * v4[2] + v1[3] * v4[4] + v1[3] * v4[5] + v1[5] * v4[1] + v1[5] * v4[3] -
-           (R)2 * v1[5] * v4[0] + v3[4] * v2[1] + (R)2 * v3[0] * v2[5] + v3[3] * v2[5] + v3[5] * v2[1] -
-           (R)2 * v3[2] * v2[1] + v3[1] * v2[5];
+    g[0] = terms(v1[2], v4[5], -v1[2], v4[4], v1[0], v4[3], -v1[0], v4[1], v3[3], v2[0], v3[5], v2[2],
+                 -v3[4], v2[2], -v3[1], v2[0]);
+    g[1] = terms(v1[1], v4[3], (R)2 * v1[4], v4[2], -v1[4], v4[4], v1[1], v4[1], -((R)2 * v1[1]), v4[0],
+                 -v1[4], v4[5], -((R)2 * v3[2]), v2[5], -v3[5], v2[5], v3[3], v2[1], -((R)2 * v3[0]), v2[1],
+                 v3[1], v2[1], -v3[4], v2[5]);
+    g[2] = terms(v1[2], v4[3], -v1[0], v4[5], v1[0], v4[4], -v1[2], v4[1], -v3[5], v2[0], v3[3], v2[2],
+                 v3[4], v2[0], -v3[1], v2[2]);
+    g[3] = terms((R)2 * v1[3], v4[0], -v1[5], v4[5], v1[3], v4[1], -v1[5], v4[4], -((R)2 * v1[5]), v4[2],
+                 v1[3], v4[3], (R)2 * v3[2], v2[4], (R)2 * v3[0], v2[3], v3[1], v2[3], -v3[5], v2[4],
+                 v3[3], v2[3], -v3[4], v2[4]);
+    g[4] = terms(v1[4], v4[1], v1[4], v4[3], (R)2 * v1[4], v4[0], v1[1], v4[4], (R)2 * v1[1], v4[2],
+                 v1[1], v4[5], v3[4], v2[3], (R)2 * v3[2], v2[3], v3[3], v2[4], v3[1], v2[4],
+                 -((R)2 * v3[0]), v2[4], v3[5], v2[3]);
+    g[5] = terms(v1[3], v4[4], -((R)2 * v1[3]), v4[2], v1[3], v4[5], v1[5], v4[1], v1[5], v4[3],
+                 -((R)2 * v1[5]), v4[0], v3[4], v2[1], (R)2 * v3[0], v2[5], v3[3], v2[5], v3[5], v2[1],
+                 -((R)2 * v3[2]), v2[1], v3[1], v2[5]);
 }
 
 // vertex component c of one slot at one site (single value), for the t-channel local vertices
@@ -140,17 +162,21 @@ __device__ __forceinline__ R gather_one(const PassArgs<R>& A, const NodeScratch<
         const int cs = comp_read(P, C, c, sgn);
         const R* q = CS == 2 ? src + c + 2 * P.base : src + P.base + cs * A.L.comp;
         const int st = P.exch ? exch_i : i;
-        R acc = P.w[0] * ldg(q + CS * (P.off[0] + st));
-        int k = 1;
+        R acc;
         if constexpr (sizeof(R) == 4 && C == 6) {
             // the second product of a bosonic pair is rounded first: the FP32 results stay those of the
             // uncompacted plan, in which the compiler chose this order (either is as exact)
+            int k = 1;
+            acc = mul_rn(P.w[0], ldg(q + P.off[0] + st));
             if (P.flags & 8) {
-                acc = fmaf(P.w[0], ldg(q + P.off[0] + st), __fmul_rn(P.w[1], ldg(q + P.off[1] + st)));
+                acc = fma(P.w[0], ldg(q + P.off[0] + st), mul_rn(P.w[1], ldg(q + P.off[1] + st)));
                 k = 2;
             }
+            for (; k < nc; ++k) acc = fma(P.w[k], ldg(q + P.off[k] + st), acc);
+        } else {
+            acc = P.w[0] * ldg(q + CS * (P.off[0] + st));
+            for (int k = 1; k < nc; ++k) acc += P.w[k] * ldg(q + CS * (P.off[k] + st));
         }
-        for (; k < nc; ++k) acc += P.w[k] * ldg(q + CS * (P.off[k] + st));
         val += sgn * acc;
     }
     return val;
@@ -286,6 +312,7 @@ struct Team {
     int tl;                 // lane in team
     int site_ex[SPL];       // exchange[site] of this lane's sites
     unsigned long long nodes, alg;
+    bool odd_first = false;  // FP32 U(1)-DM: see eval_u1dm
 
     // offset of the first kernel of the s channel in a vertex source
     __device__ __forceinline__ int64_t q0() const {
@@ -372,20 +399,21 @@ struct Team {
             __syncwarp();
             if (X == 1) eval_t_overlap(count, sink);
             __syncwarp();
-            return;
-        }
-        // phase B of U(1)-DM: gathers and per-site combination, node by node
-        for (int j = 0; j < mx; ++j) {
-            const bool act = j < count;
-            const NodeScratch<R, C>& ns = ts.node[act ? j : 0];
-            R p = (R)0;
-            R v1[C][SPL], v2[C][SPL];
-            if (act) {
-                p = ns.p;
-                gather_slot<R, T, SPL, C>(A, ns, 0, tl, site_ex, v1);
-                gather_slot<R, T, SPL, C>(A, ns, 1, tl, site_ex, v2);
+        } else {
+            // phase B of U(1)-DM: gathers and per-site combination, node by node
+#pragma unroll 1
+            for (int j = 0; j < mx; ++j) {
+                const bool act = j < count;
+                const NodeScratch<R, C>& ns = ts.node[act ? j : 0];
+                R p = (R)0;
+                R v1[C][SPL], v2[C][SPL];
+                if (act) {
+                    p = ns.p;
+                    gather_slot<R, T, SPL, C>(A, ns, 0, tl, site_ex, v1);
+                    gather_slot<R, T, SPL, C>(A, ns, 1, tl, site_ex, v2);
+                }
+                eval_u1dm(X, j, act, p, ns, v1, v2, sink);
             }
-            eval_u1dm(X, j, act, p, ns, v1, v2, sink);
         }
     }
 
@@ -618,9 +646,8 @@ struct Team {
         }
         __syncwarp(team_mask);
         const R twoS = (R)A.twoS;
-#pragma unroll
-        for (int jj = 0; jj < NB; ++jj) {
-            if (jj >= count) continue;
+#pragma unroll 1
+        for (int jj = 0; jj < count; ++jj) {
             const NodeScratch<R, C>& ns = ts.node[jj];
             const R p = ns.p;
             const R coef = -p * (R)-2 * twoS;
@@ -683,15 +710,32 @@ struct Team {
             sink(j, g);
         }
         const bool tch = act && X == 1;
+        // both slots of a site lie in 16-byte pieces (FP32: four and two components, FP64 three pairs), so a
+        // row of the overlap sum takes two or three loads per slot instead of six (with the FP64 form below,
+        // kagome L = 8 three loops mixed 252 -> 247 ms, kagome L = 3 FP64 25.2 -> 24.8 ms)
+        using V4 = typename std::conditional<sizeof(R) == 4, float4, double2>::type;
+        using V2 = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
+        V4* t1a = reinterpret_cast<V4*>(tmp);
+        V4* t2a = t1a + (sizeof(R) == 4 ? Ns : 2 * Ns);
+        V2* t1b = reinterpret_cast<V2*>(t2a + (sizeof(R) == 4 ? Ns : 2 * Ns));
+        V2* t2b = t1b + Ns;
         if (tch) {
 #pragma unroll
             for (int k = 0; k < SPL; ++k) {
                 const int i = tl + k * T;
                 if (i < Ns) {
-#pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        tmp[c * Ns + i] = v1[c][k];
-                        tmp[(C + c) * Ns + i] = v2[c][k];
+                    if constexpr (sizeof(R) == 4) {
+                        t1a[i] = make_float4(v1[0][k], v1[1][k], v1[2][k], v1[3][k]);
+                        t2a[i] = make_float4(v2[0][k], v2[1][k], v2[2][k], v2[3][k]);
+                        t1b[i] = make_float2(v1[4][k], v1[5][k]);
+                        t2b[i] = make_float2(v2[4][k], v2[5][k]);
+                    } else {
+                        t1a[i] = make_double2(v1[0][k], v1[1][k]);
+                        t1a[Ns + i] = make_double2(v1[2][k], v1[3][k]);
+                        t2a[i] = make_double2(v2[0][k], v2[1][k]);
+                        t2a[Ns + i] = make_double2(v2[2][k], v2[3][k]);
+                        t1b[i] = make_double2(v1[4][k], v1[5][k]);
+                        t2b[i] = make_double2(v2[4][k], v2[5][k]);
                     }
                 }
             }
@@ -710,24 +754,76 @@ struct Team {
                     b[c] = v2[c][k];
                 }
                 u1dm_t(a, b, ns.loc, ns.loc + C, G);
+                // overlap sum (flow_u1_dm_t.jl:86-110)
+                int r = 0, j1 = 0;
+                if (i < Ns) r = row_off[i], j1 = row_off[i + 1];
+                if constexpr (sizeof(R) == 4) {
+                    // one row: the six bilinear terms of its two sites
+                    auto row_terms = [&](unsigned row, R* x) {
+                        const int ia = row & 0xff, ib = (row >> 8) & 0xff;
+                        const float4 p1 = t1a[ia], p2 = t2a[ib];
+                        const float2 q1 = t1b[ia], q2 = t2b[ib];
+                        x[0] = terms(p1.x, p2.x, -p1.z, p2.z);
+                        x[1] = terms(p1.y, p2.y, -q1.x, q2.y);
+                        x[2] = terms(p1.z, p2.x, p1.x, p2.z);
+                        x[3] = terms(p1.w, p2.w, -q1.y, q2.x);
+                        x[4] = terms(q1.x, p2.w, p1.y, q2.x);
+                        x[5] = terms(p1.w, q2.y, q1.y, p2.y);
+                    };
+                    // refining nodes of lattices with three sites per lane: the first of an odd number of rows is
+                    // fused with the local part's factor, as a compiler unrolled these loops once; either order is
+                    // as exact, and FP32 results stay what they were
+                    const bool odd = odd_first && k < 2 && ((j1 - r) & 1);
+                    if (odd) {
+                        R x[C];
+                        row_terms(rows[r], x);
+                        const R mm = coef * (R)(rows[r] >> 16);
 #pragma unroll
-                for (int c = 0; c < C; ++c) G[c] = -p * G[c];
-                if (i < Ns) {
-                    // overlap sum (flow_u1_dm_t.jl:86-110)
-                    const int j0 = row_off[i], j1 = row_off[i + 1];
-                    for (int r = j0; r < j1; ++r) {
+                        for (int c = 0; c < C; ++c) G[c] = fma(-p, G[c], mul_rn(mm, x[c]));
+                        ++r;
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < C; ++c) G[c] = mul_rn(-p, G[c]);
+                    }
+#pragma unroll 2
+                    for (; r < j1; ++r) {
+                        const unsigned row = rows[r];
+                        R x[C];
+                        row_terms(row, x);
+                        const R mm = coef * (R)(row >> 16);
+#pragma unroll
+                        for (int c = 0; c < C; ++c) G[c] = fma(mm, x[c], G[c]);
+                    }
+                } else {
+                    // FP64: twelve multiply-adds a row; the common factor comes last, and the multiplicity,
+                    // which is one for nearly all rows, only where it counts (19 FP64 operations with both in
+                    // every row)
+                    R S[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+                    for (; r < j1; ++r) {
                         const unsigned row = rows[r];
                         const int ia = row & 0xff, ib = (row >> 8) & 0xff;
-                        const R mm = coef * (R)(row >> 16);
-                        const R* t1 = tmp + ia;
-                        const R* t2 = tmp + C * Ns + ib;
-                        G[0] += mm * (t1[0] * t2[0] - t1[2 * Ns] * t2[2 * Ns]);
-                        G[1] += mm * (t1[Ns] * t2[Ns] - t1[4 * Ns] * t2[5 * Ns]);
-                        G[2] += mm * (t1[2 * Ns] * t2[0] + t1[0] * t2[2 * Ns]);
-                        G[3] += mm * (t1[3 * Ns] * t2[3 * Ns] - t1[5 * Ns] * t2[4 * Ns]);
-                        G[4] += mm * (t1[4 * Ns] * t2[3 * Ns] + t1[Ns] * t2[4 * Ns]);
-                        G[5] += mm * (t1[3 * Ns] * t2[5 * Ns] + t1[5 * Ns] * t2[Ns]);
+                        double2 x01 = t1a[ia], x23 = t1a[Ns + ia], x45 = t1b[ia];
+                        const double2 y01 = t2a[ib], y23 = t2a[Ns + ib], y45 = t2b[ib];
+                        if ((row >> 16) != 1) {
+                            const R m = (R)(row >> 16);
+                            x01.x *= m, x01.y *= m, x23.x *= m, x23.y *= m, x45.x *= m, x45.y *= m;
+                        }
+                        S[0] = fma(x01.x, y01.x, S[0]);
+                        S[1] = fma(x01.y, y01.y, S[1]);
+                        S[2] = fma(x23.x, y01.x, S[2]);
+                        S[3] = fma(x23.y, y23.y, S[3]);
+                        S[4] = fma(x45.x, y23.y, S[4]);
+                        S[5] = fma(x23.y, y45.y, S[5]);
+                        S[0] = fma(-x23.x, y23.x, S[0]);
+                        S[1] = fma(-x45.x, y45.y, S[1]);
+                        S[2] = fma(x01.x, y23.x, S[2]);
+                        S[3] = fma(-x45.y, y45.x, S[3]);
+                        S[4] = fma(x01.y, y45.x, S[4]);
+                        S[5] = fma(x45.y, y01.y, S[5]);
                     }
+#pragma unroll
+                    for (int c = 0; c < C; ++c) G[c] = fma(coef, S[c], -p * G[c]);
                 }
 #pragma unroll
                 for (int c = 0; c < C; ++c) g[c][k] = G[c];
@@ -765,7 +861,7 @@ struct LevelCut {
 // steps, coarse cut only against this rule: square L = 3 11/4/3 FP64 40.1 -> 18.8 ms and 50/15/10 mixed
 // 34.1 -> 22.1 ms, kagome L = 8 U(1)-DM three loops mixed 482 -> 293 ms, honeycomb L = 5 two-loop step mixed
 // 222 -> 167 ms, pyrochlore L = 6 two loops mixed 377 -> 351 ms.
-__host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, int batch, int teams) {
+__host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, int batch, int least, int teams) {
     LevelCut k;
     const int per0 = n <= (long long)kChunk * kMaxChunks ? (int)(n < kChunk ? n : kChunk) : (int)(n / kMaxChunks);
     k.coarse = (int)(n / per0);
@@ -779,7 +875,25 @@ __host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, i
         k.per >>= 1;
         k.chunks <<= 1;
     }
+    // U(1)-DM batches, whose nodes are evaluated one by one (least = 1), are halved further while an SM has
+    // less than a block's teams; SU(2) batches share the overlap rows and the setup
+    const long long few = most < teams / 8 ? most : teams / 8;
+    while (k.per > least && 2ll * k.nact * k.chunks <= few) {
+        k.per >>= 1;
+        k.chunks <<= 1;
+    }
     return k;
+}
+
+// Blocks of eval_kernel that work on nchunks chunks (npw teams per warp).  With fewer warps' worth of
+// chunks than fill a block on every SM, one block per SM takes them in turn, so that the work spreads over
+// the SMs' FP64 pipes and caches; otherwise the warps of a block take neighbouring chunks, which share
+// vertex rows.
+constexpr int kSMs = 152;
+__host__ __device__ inline int eval_blocks(int nchunks, int npw) {
+    const int units = (nchunks + npw - 1) / npw;
+    const int full = (units + kWarps - 1) / kWarps;
+    return full > kSMs ? full : (units < kSMs ? units : kSMs);
 }
 
 // per-site sums of |node values| of the fine chunks of a level (FP32 pass of the mixed path): vectors
@@ -929,28 +1043,57 @@ __device__ __forceinline__ bool sub_range(const PassArgs<R>& A, const TaskInfo& 
     return true;
 }
 
-// the reference's convergence test of simps! on one team's sites; returns 1 when done
-template <int T, int SPL, int C>
-__device__ __forceinline__ int simps_test(const double s_old[C][SPL], const double s_new[C][SPL], long long n,
-                                          double atol, double rtol, int team, bool in_team0_only) {
-    double ss_r = 0.0, ss_n = 0.0, ss_d = 0.0;
+// Norms of a team's per-site values: x[q] is this lane's sum of squares of quantity q, on return the
+// norm over the team's sites in every lane.  The lanes halve the quantities they carry at every step of the
+// sum (7 to 9 FP64 additions instead of 6 log2 T), so each ends with one total and takes one square root for
+// all quantities (an FP64 square root costs a warp as much as some fifteen additions).
+constexpr int kNorms = 8;
+template <int T>
+__device__ __forceinline__ void team_norms(double x[kNorms]) {
+    const int tl = threadIdx.x & (T - 1);
+    int n = kNorms;
+#pragma unroll
+    for (int o = T / 2; o >= 1; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = (tl & o) != 0;
+#pragma unroll
+            for (int k = 0; k < kNorms / 2; ++k)
+                if (k < n) {
+                    const double send = up ? x[k] : x[k + n];
+                    const double keep = up ? x[k + n] : x[k];
+                    x[k] = keep + __shfl_xor_sync(kFull, send, o);
+                }
+        } else {
+            x[0] += __shfl_xor_sync(kFull, x[0], o);
+        }
+    }
+    // lane tl holds the quantity of its top three bits
+    const double r = sqrt(x[0]);
+#pragma unroll
+    for (int q = 0; q < kNorms; ++q) x[q] = __shfl_sync(kFull, r, q * (T / kNorms), T);
+}
+
+// this lane's sums of squares of the convergence test of simps!: x[0] the Richardson value R, x[1] the new
+// Simpson sum S, x[2] R - S
+template <int SPL, int C>
+__device__ __forceinline__ void simps_squares(const double s_old[C][SPL], const double s_new[C][SPL], double* x) {
+    x[0] = x[1] = x[2] = 0.0;
 #pragma unroll
     for (int c = 0; c < C; ++c)
 #pragma unroll
         for (int k = 0; k < SPL; ++k) {
             const double rich = s_old[c][k] * (-1.0 / 15.0) + (16.0 / 15.0) * s_new[c][k];
             const double dd = rich - s_new[c][k];
-            ss_r += rich * rich;
-            ss_n += s_new[c][k] * s_new[c][k];
-            ss_d += dd * dd;
+            x[0] += rich * rich;
+            x[1] += s_new[c][k] * s_new[c][k];
+            x[2] += dd * dd;
         }
-    (void)team;
-    (void)in_team0_only;
-    ss_r = in_team_sum<T>(ss_r);
-    ss_n = in_team_sum<T>(ss_n);
-    ss_d = in_team_sum<T>(ss_d);
-    const double adiff = sqrt(ss_d);
-    const double rdiff = adiff / fmax(sqrt(ss_r), sqrt(ss_n));
+}
+
+// the reference's convergence test of simps!, from the norms of R, S and R - S; 1 when done
+__device__ __forceinline__ int simps_test(double nr, double ns, double adiff, long long n, double atol, double rtol) {
+    const double rdiff = adiff / fmax(nr, ns);
     // a non-finite integrand stops refining at once (the reference would refine it to n > 2^20);
     // the result's finite check then reports it
     return (adiff < atol || rdiff < rtol || 2 * n > (1ll << 20) || !isfinite(adiff)) ? 1 : 0;
@@ -962,25 +1105,9 @@ __device__ __forceinline__ int simps_test(const double s_old[C][SPL], const doub
 // within eps sa of the FP32 ones, so when the test is closer to one of its bounds than that
 // margin the FP64 evaluation of the same nodes could decide the other way, and the subdomain is
 // evaluated again in FP64 from its first level (all its decisions then are the FP64 path's).
-template <int T, int SPL, int C>
-__device__ __forceinline__ int simps_decide(const double s_old[C][SPL], const double s_new[C][SPL], long long n,
-                                            double atol, double rtol, double eps, double sa_old, double sa_new) {
-    double ss_r = 0.0, ss_n = 0.0, ss_d = 0.0;
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-#pragma unroll
-        for (int k = 0; k < SPL; ++k) {
-            const double rich = s_old[c][k] * (-1.0 / 15.0) + (16.0 / 15.0) * s_new[c][k];
-            const double dd = rich - s_new[c][k];
-            ss_r += rich * rich;
-            ss_n += s_new[c][k] * s_new[c][k];
-            ss_d += dd * dd;
-        }
-    ss_r = in_team_sum<T>(ss_r);
-    ss_n = in_team_sum<T>(ss_n);
-    ss_d = in_team_sum<T>(ss_d);
-    const double adiff = sqrt(ss_d);
-    const double den = fmax(sqrt(ss_r), sqrt(ss_n));
+__device__ __forceinline__ int simps_decide(double nr, double ns, double adiff, long long n, double atol, double rtol,
+                                            double eps, double sa_old, double sa_new) {
+    const double den = fmax(nr, ns);
     if (2 * n > (1ll << 20) || !isfinite(adiff)) return 1;
     const int done = (adiff < atol || adiff / den < rtol) ? 1 : 0;
     const double E = eps * (sa_new + sa_old) / 15.0;          // |Δ64 - Δ32|
@@ -1007,8 +1134,14 @@ __device__ __forceinline__ void hand_off(WaveSpace& Wsp, int sub) {
 }
 
 // ---- wave 0: first five nodes of every subdomain, boundary nodes, first test ----
+// (blocks per SM that SU(2) kernels with at most two sites per lane are held to: FP32 three, four and five
+// blocks 226, 217 and 222 ms summed over two honeycomb L = 5 steps; FP64 with two sites per lane three, four
+// blocks 99.0, 100.0 ms on pyrochlore L = 6, with one site 33.8, 33.3 ms on a honeycomb L = 4 parquet solve)
+template <typename R, int SPL, int C>
+constexpr int wave0_min_blocks() { return C == 2 && SPL <= 2 ? (sizeof(R) == 4 || SPL == 1 ? 4 : 3) : 1; }
+
 template <typename R, int T, int SPL, int C>
-__global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveSpace Wsp) {
+__global__ void __launch_bounds__(kWarps * 32, wave0_min_blocks<R, SPL, C>()) wave0_kernel(PassArgs<R> A, WaveSpace Wsp) {
     constexpr int NPW = 32 / T;
     extern __shared__ __align__(16) unsigned char smem[];
     load_common<R, T, C, SPL>(A, smem);
@@ -1055,61 +1188,96 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
         }
         typename Team<R, T, SPL, C>::SetupT W(0.0), V(0.0), VP(0.0);
         if (valid) task_freqs(A, M, ti, W, V, VP);
+        // simps!: 3-point sum s_old, 5-point sum s_new via residual! with n = 2 from the new nodes' sum f and
+        // the middle node, Richardson test; boundary nodes are summed with their corrections into s_old.
+        // FP32 kernels add a node's values as they come: kept until the end, five nodes' values sat in local
+        // memory (two honeycomb L = 5 steps 235 -> 218 ms with this and one square root per test); the FP64
+        // kernels, bound by their FP64 operations, measured the same either way and keep them.
+        const bool simpson = valid && !boundary && cnt == 5;
+        const double we = 1.0 * (hi - lo) / 6.0, wm = 2.0 * (hi - lo) / 3.0;
+        constexpr int CA = sizeof(R) == 4 ? C : 1;  // sums over |node values|: FP32 pass of the mixed path
+        double s_old[C][SPL], f_new[C][SPL], a_old[CA][SPL], a_f[CA][SPL];
+        R g2[C][SPL], g5[sizeof(R) == 8 ? 5 : 1][C][SPL];
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int k = 0; k < SPL; ++k) {
+                s_old[c][k] = f_new[c][k] = 0.0;
+                g2[c][k] = (R)0;
+                if (c < CA) a_old[c][k] = a_f[c][k] = 0.0;
+            }
         // all teams of the warp evaluate together (cnt = 0 for idle teams), NB nodes at a time
-        R g[5][C][SPL];
 #pragma unroll 1
         for (int b = 0; b < 5; b += NB) {
             const int nb = max(0, min(NB, cnt - b));
             for (int j = tl; j < nb; j += T) tm.ts.node[j].x = x[b + j];
             __syncwarp();
-            auto keep = [&](int j, const R (&gv)[C][SPL]) {
+            auto add = [&](int j, const R (&gv)[C][SPL]) {
+                const int q = b + j;
+                const bool mid = !boundary && (q & 1);
+                const double w = boundary ? (q == 0 ? c0 : c1) : (q == 2 ? wm : we);
 #pragma unroll
                 for (int c = 0; c < C; ++c)
 #pragma unroll
-                    for (int k = 0; k < SPL; ++k) g[b + j][c][k] = gv[c][k];
+                    for (int k = 0; k < SPL; ++k) {
+                        if constexpr (sizeof(R) == 4) {
+                            const double g = (double)gv[c][k];
+                            if (mid) {
+                                f_new[c][k] += g;
+                                a_f[c][k] += fabs(g);
+                            } else {
+                                s_old[c][k] += w * g;
+                                a_old[c][k] += w * fabs(g);
+                            }
+                            if (q == 2) g2[c][k] = gv[c][k];
+                        } else {
+                            g5[q][c][k] = gv[c][k];
+                        }
+                    }
             };
-            tm.eval(ti, W, V, VP, nb, keep);
+            tm.eval(ti, W, V, VP, nb, add);
         }
-        const bool simpson = valid && !boundary && cnt == 5;
-        // simps!: 3-point sum, 5-point sum via residual! with n = 2, Richardson test
-        const double we = 1.0 * (hi - lo) / 6.0, wm = 2.0 * (hi - lo) / 3.0;
         const double h = 0.5 * (hi - lo) / 2.0;
         const double wn = 4.0 * h / 3.0, wo = -2.0 * h / 3.0;
-        double s_old[C][SPL], s_new[C][SPL], f_new[C][SPL];
+        double s_new[C][SPL], nx[kNorms];
 #pragma unroll
         for (int c = 0; c < C; ++c)
 #pragma unroll
             for (int k = 0; k < SPL; ++k) {
-                s_old[c][k] = s_new[c][k] = f_new[c][k] = 0.0;
-                if (!simpson) continue;
-                s_old[c][k] = we * (double)g[0][c][k];
-                s_old[c][k] += wm * (double)g[2][c][k];
-                s_old[c][k] += we * (double)g[4][c][k];
-                f_new[c][k] = (double)g[1][c][k] + (double)g[3][c][k];
-                s_new[c][k] = 0.5 * s_old[c][k] + wn * f_new[c][k] + wo * (double)g[2][c][k];
+                if constexpr (sizeof(R) == 8) {
+                    s_old[c][k] = s_new[c][k] = f_new[c][k] = 0.0;
+                    if (!simpson) continue;
+                    s_old[c][k] = we * g5[0][c][k];
+                    s_old[c][k] += wm * g5[2][c][k];
+                    s_old[c][k] += we * g5[4][c][k];
+                    f_new[c][k] = g5[1][c][k] + g5[3][c][k];
+                    s_new[c][k] = 0.5 * s_old[c][k] + wn * f_new[c][k] + wo * g5[2][c][k];
+                } else {
+                    s_new[c][k] = 0.5 * s_old[c][k] + wn * f_new[c][k] + wo * (double)g2[c][k];
+                }
             }
         // every lane takes part in the test's team reductions
         int done;
         double sa_new = 0.0, fab = 0.0;
-        if (A.esc_mode == 1) {
-            double a_old[C][SPL], a_new[C][SPL], a_f[C][SPL];
+        simps_squares<SPL, C>(s_old, s_new, nx);
+        nx[3] = nx[4] = nx[5] = nx[6] = nx[7] = 0.0;
+        if (sizeof(R) == 4 && A.esc_mode == 1) {
 #pragma unroll
-            for (int c = 0; c < C; ++c)
+            for (int c = 0; c < CA; ++c)
 #pragma unroll
                 for (int k = 0; k < SPL; ++k) {
-                    a_old[c][k] = a_new[c][k] = a_f[c][k] = 0.0;
-                    if (!simpson) continue;
-                    a_old[c][k] = we * fabs((double)g[0][c][k]) + wm * fabs((double)g[2][c][k]) +
-                                  we * fabs((double)g[4][c][k]);
-                    a_f[c][k] = fabs((double)g[1][c][k]) + fabs((double)g[3][c][k]);
-                    a_new[c][k] = 0.5 * a_old[c][k] + fabs(wn) * a_f[c][k] + fabs(wo) * fabs((double)g[2][c][k]);
+                    const double a_new = 0.5 * a_old[c][k] + fabs(wn) * a_f[c][k] + fabs(wo) * fabs((double)g2[c][k]);
+                    nx[3] += a_old[c][k] * a_old[c][k];
+                    nx[4] += a_new * a_new;
+                    nx[5] += a_f[c][k] * a_f[c][k];
                 }
-            const double sa_old = team_norm<T, SPL, C>(a_old);
-            sa_new = team_norm<T, SPL, C>(a_new);
-            fab = team_norm<T, SPL, C>(a_f);
-            done = simps_decide<T, SPL, C>(s_old, s_new, 2, A.atol, A.rtol, A.esc_eps, sa_old, sa_new);
+            team_norms<T>(nx);
+            sa_new = nx[4];
+            fab = nx[5];
+            done = simps_decide(nx[0], nx[1], nx[2], 2, A.atol, A.rtol, A.esc_eps, nx[3], sa_new);
         } else {
-            done = simps_test<T, SPL, C>(s_old, s_new, 2, A.atol, A.rtol, team, false);
+            team_norms<T>(nx);
+            done = simps_test(nx[0], nx[1], nx[2], 2, A.atol, A.rtol);
         }
         if (!valid) continue;
         if (simpson && done == 2) {
@@ -1125,7 +1293,9 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
 #pragma unroll
                 for (int k = 0; k < SPL; ++k) {
                     const int i = tl + k * T;
-                    if (i < Ns) sA[c * Ns + i] = boundary ? c0 * (double)g[0][c][k] + c1 * (double)g[1][c][k] : 0.0;
+                    if (i >= Ns) continue;
+                    if constexpr (sizeof(R) == 4) sA[c * Ns + i] = boundary ? s_old[c][k] : 0.0;
+                    else sA[c * Ns + i] = boundary ? c0 * g5[0][c][k] + c1 * g5[1][c][k] : 0.0;
                 }
             continue;
         }
@@ -1156,12 +1326,12 @@ __global__ void __launch_bounds__(kWarps * 32) wave0_kernel(PassArgs<R> A, WaveS
 }
 
 // ---- wave k >= 1: evaluate queued chunks, one partial node sum per chunk ----
-// (FP32 kernels: SU(2) teams with at most two sites per lane held to 128 registers, four blocks of 128
-// threads per SM, where their gathers do not spill (3-5 % faster than three blocks on the pyrochlore L = 6
-// and square L = 5, 8 states); wider lanes and U(1)-DM entries, whose gathers spill at 128, held to 168
-// registers, three blocks)
+// (FP32 kernels: SU(2) teams with one site per lane held to 102 registers, five blocks of 128 threads per SM
+// (four, five and six blocks 11.0, 10.5 and 10.8 ms summed over two square L = 3 right-hand sides), with two
+// sites to 128, four blocks (their gathers spill beyond that); wider lanes and U(1)-DM entries, whose gathers
+// spill at 128, to 168, three blocks)
 template <typename R, int T, int SPL, int C>
-constexpr int eval_min_blocks() { return sizeof(R) == 4 ? (C == 2 && SPL <= 2 ? 4 : 3) : 1; }
+constexpr int eval_min_blocks() { return sizeof(R) == 4 ? (C == 2 && SPL <= 2 ? (SPL == 1 ? 5 : 4) : 3) : 1; }
 
 template <typename R, int T, int SPL, int C>
 __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
@@ -1170,7 +1340,7 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
     constexpr int NB = BatchOf<T, C, SPL>::NB;
     extern __shared__ __align__(16) unsigned char smem[];
     const int nactive = Wsp.counters[2 + par];
-    const LevelCut K = cut_level(nactive, n, Wsp.qcap, NB, Wsp.teams);
+    const LevelCut K = cut_level(nactive, n, Wsp.qcap, NB, C == 6 ? 1 : NB, Wsp.teams);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // the next level's list starts empty (this wave's decide_kernel fills it)
         Wsp.counters[2 + (par ^ 1)] = 0;
@@ -1179,17 +1349,21 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
     }
     const int nchunks = K.nact * K.chunks;
     // blocks without a chunk leave before staging the meshes and rows
-    if ((long long)blockIdx.x * kWarps * NPW >= nchunks) return;
+    const int nblocks = min((int)gridDim.x, eval_blocks(nchunks, NPW));
+    if ((int)blockIdx.x >= nblocks) return;
     load_common<R, T, C, SPL>(A, smem);
     const auto M = setup_mesh(A, smem);  // staged in shared memory by load_common
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int team = lane / T, tl = lane % T;
     Team<R, T, SPL, C> tm = make_team<R, T, SPL, C>(A, smem, M, warp, team, tl);
+    tm.odd_first = SPL == 3;
     const int Ns = A.L.Ns;
     const int jobs = 4 * A.eval + 1;
     const int* active = par ? Wsp.active[1] : Wsp.active[0];
-    const long long nwarps = (long long)gridDim.x * kWarps;
-    for (long long base = ((long long)blockIdx.x * kWarps + warp) * NPW; base < nchunks; base += nwarps * NPW) {
+    const bool spread = nblocks <= kSMs;  // unit of NPW chunks of this warp: in turn, or a block's warps together
+    const long long nwarps = (long long)nblocks * kWarps;
+    for (long long base = (long long)(spread ? warp * nblocks + blockIdx.x : blockIdx.x * kWarps + warp) * NPW;
+         base < nchunks; base += nwarps * NPW) {
         const int chunk = (int)(base + team);
         const bool valid = chunk < nchunks;
         int first = 0;  // first new node of the chunk
@@ -1290,7 +1464,8 @@ __global__ void __launch_bounds__(kWarps * 32) decide_kernel(WaveSpace Wsp, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int team = lane / T, tl = lane % T;
     const int bteam = warp * NPW + team;
-    const LevelCut K = cut_level(Wsp.counters[2 + par], n, Wsp.qcap, BatchOf<T, C, SPL>::NB, Wsp.teams);
+    const LevelCut K = cut_level(Wsp.counters[2 + par], n, Wsp.qcap, BatchOf<T, C, SPL>::NB,
+                                 C == 6 ? 1 : BatchOf<T, C, SPL>::NB, Wsp.teams);
     const int* active = par ? Wsp.active[1] : Wsp.active[0];
     const bool split = K.chunks >= kDecideSplit;
     const int G = split ? TPB : 1, g = split ? bteam : 0;
@@ -1380,13 +1555,16 @@ __global__ void __launch_bounds__(kWarps * 32) decide_kernel(WaveSpace Wsp, int 
                 s_new[c][k] = 0.5 * s_old[c][k] + wn * f_new[c][k] + wo * sB[c * Ns + i];
             }
         int done;
-        double sa_new = 0.0;
+        double sa_new = 0.0, nx[kNorms];
+        simps_squares<SPL, C>(s_old, s_new, nx);
+        nx[3] = nx[4] = nx[5] = nx[6] = nx[7] = 0.0;
+        team_norms<T>(nx);
         if (esc_mode == 1) {
             const double sa_old = S.sa;
             sa_new = 0.5 * sa_old + fabs(wn) * fa_new + fabs(wo) * S.fab;
-            done = simps_decide<T, SPL, C>(s_old, s_new, n, atol, rtol, esc_eps, sa_old, sa_new);
+            done = simps_decide(nx[0], nx[1], nx[2], n, atol, rtol, esc_eps, sa_old, sa_new);
         } else {
-            done = simps_test<T, SPL, C>(s_old, s_new, n, atol, rtol, team, false);
+            done = simps_test(nx[0], nx[1], nx[2], n, atol, rtol);
         }
         if (!valid || (split && team > 0)) continue;
         if (done == 2) {
@@ -1477,7 +1655,7 @@ struct PassLauncher {
         const int teams_per_block = kWarps * NPW;
         // the FP64 pass of the mixed path keeps the count of handed subdomains (counters[5])
         if ((e = cudaMemsetAsync(Wsp.counters, 0, sizeof(int) * (a.esc_mode == 2 ? 5 : 6), st))) return e;
-        Wsp.teams = 2 * 4 * 152 * teams_per_block;  // twice the teams of four blocks per SM
+        Wsp.teams = 2 * 4 * kSMs * teams_per_block;  // twice the teams of four blocks per SM
         int g0 = (Wsp.nsub + teams_per_block - 1) / teams_per_block;
         // h_counters[7] counts the kernels this pass launches
         wave0_kernel<R, T, SPL, C><<<g0 < grid_cap ? g0 : grid_cap, kWarps * 32, smem, st>>>(a, Wsp);
@@ -1512,12 +1690,13 @@ struct PassLauncher {
             if ((e = cudaStreamSynchronize(st))) return e;
             const int nact = h_counters[2 + par];
             if (nact == 0) break;
-            const LevelCut K = cut_level(nact, 2ll << wave, Wsp.qcap, BatchOf<T, C, SPL>::NB, Wsp.teams);
+            const LevelCut K = cut_level(nact, 2ll << wave, Wsp.qcap, BatchOf<T, C, SPL>::NB,
+                                 C == 6 ? 1 : BatchOf<T, C, SPL>::NB, Wsp.teams);
             if (K.overflow) {  // chunk queue overflow
                 h_counters[4] = 1;
                 return cudaErrorLaunchOutOfResources;
             }
-            int ge = (K.nact * K.chunks + teams_per_block - 1) / teams_per_block;
+            const int ge = eval_blocks(K.nact * K.chunks, NPW);
             eval_kernel<R, T, SPL, C><<<ge < grid_cap ? ge : grid_cap, kWarps * 32, smem, st>>>(a, Wsp, par, 2ll << wave);
             h_counters[7] += 2;
             if ((e = cudaGetLastError())) return e;

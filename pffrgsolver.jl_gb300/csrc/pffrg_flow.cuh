@@ -590,34 +590,70 @@ struct Team {
         const unsigned team_mask = (T == 32) ? kFull : (((1u << T) - 1u) << ((threadIdx.x & 31) / T * T));
         constexpr int V = 2 * NB;  // sums per site: (spin, density) of every node of the batch
         R* ovr = reinterpret_cast<R*>(ov);
+        // FP32 teams of a warp fetch the next row while one is worked on, across the end of a site's list too:
+        // long lists do not fit in shared memory beside the staging and are read through L1, of which the
+        // vertex gathers leave little (pyrochlore L = 6 two loops mixed 249 -> 235 ms; narrower teams, whose
+        // short lists stay in shared memory, were 1.5 % slower with it).
+        constexpr bool kAhead = sizeof(R) == 4 && T == 32;
+        int r = tl, j1 = row_off[0], rn = j1 + tl;
+        const int last = row_off[Ns] - 1;
+        unsigned next = kAhead && last >= 0 ? rows[min(rn, last)] : 0;
         for (int i = 0; i < Ns; ++i) {
             R x[V];
 #pragma unroll
             for (int v = 0; v < V; ++v) x[v] = (R)0;
-            const int j1 = row_off[i + 1];
+            r = j1 + tl;
+            j1 = row_off[i + 1];
+            if (kAhead && rn != r && r < j1) next = rows[r];  // the list before had no row for this lane
 #pragma unroll 2
-            for (int r = row_off[i] + tl; r < j1; r += T) {
-                const unsigned row = rows[r];
+            for (; r < j1; r += T) {
+                unsigned row;
+                if constexpr (kAhead) {
+                    row = next;
+                    rn = r + T < j1 ? r + T : j1 + tl;
+                    next = rows[min(rn, last)];
+                } else {
+                    row = rows[r];
+                }
                 const int ia = row & 0xff, ib = (row >> 8) & 0xff;
-                const R m = (R)(row >> 16);
                 const R2* pa = tb1 + (size_t)ia * SS;
                 const R2* pb = tb2 + (size_t)ib * SS;
+                // most rows have multiplicity one (pyrochlore L = 6: 60 % of the steps of 32 rows have no other),
+                // and in FP64 its product with the first slot is half of a row's operations (pyrochlore L = 6
+                // FP64 99 -> 79 ms); short FP32 lists multiply without looking
+                const bool scaled = (sizeof(R) == 4 && T < 32) || (row >> 16) != 1;
                 if constexpr (sizeof(R) == 4 && NB % 2 == 0) {
+                    float4 a[NB / 2];
+#pragma unroll
+                    for (int j2 = 0; j2 < NB / 2; ++j2) a[j2] = reinterpret_cast<const float4*>(pa)[j2];
+                    if (scaled) {
+                        const R m = (R)(row >> 16);
+#pragma unroll
+                        for (int j2 = 0; j2 < NB / 2; ++j2)
+                            a[j2].x = m * a[j2].x, a[j2].y = m * a[j2].y, a[j2].z = m * a[j2].z, a[j2].w = m * a[j2].w;
+                    }
 #pragma unroll
                     for (int j2 = 0; j2 < NB / 2; ++j2) {
-                        const float4 a = reinterpret_cast<const float4*>(pa)[j2];
                         const float4 b = reinterpret_cast<const float4*>(pb)[j2];
-                        x[4 * j2 + 0] += m * a.x * b.x;
-                        x[4 * j2 + 1] += m * a.y * b.y;
-                        x[4 * j2 + 2] += m * a.z * b.z;
-                        x[4 * j2 + 3] += m * a.w * b.w;
+                        x[4 * j2 + 0] = fma(a[j2].x, b.x, x[4 * j2 + 0]);
+                        x[4 * j2 + 1] = fma(a[j2].y, b.y, x[4 * j2 + 1]);
+                        x[4 * j2 + 2] = fma(a[j2].z, b.z, x[4 * j2 + 2]);
+                        x[4 * j2 + 3] = fma(a[j2].w, b.w, x[4 * j2 + 3]);
                     }
                 } else {
+                    R2 a[NB];
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) a[j] = pa[j];
+                    if (scaled) {
+                        const R m = (R)(row >> 16);
+#pragma unroll
+                        for (int j = 0; j < NB; ++j) a[j].x = m * a[j].x, a[j].y = m * a[j].y;
+                    }
 #pragma unroll
                     for (int j = 0; j < NB; ++j) {
-                        const R2 a = pa[j], b = pb[j];
-                        x[2 * j] += m * a.x * b.x;
-                        x[2 * j + 1] += m * a.y * b.y;
+                        const R2 b = pb[j];
+                        x[2 * j] = fma(a[j].x, b.x, x[2 * j]);
+                        x[2 * j + 1] = fma(a[j].y, b.y, x[2 * j + 1]);
                     }
                 }
             }

@@ -420,8 +420,9 @@ struct ChiScratch {
             unsigned cnt[kChiThreads / 32][256];
         } sort;
     };
-    // the FP64 integrand's propagator factors of a chunk's regions: [region][7 x | 7 y] coordinates
-    double gfac[kChiChunk * 14];
+    // what depends on one coordinate of the FP64 integrand, for a chunk's regions: [region][7 x | 7 y]
+    // propagator factors and frequencies
+    double gfac[kChiChunk * 14], freq[kChiChunk * 14];
     unsigned wsum[kChiThreads / 32];
     double tot_val, tot_err;
     long long numeval;
@@ -632,19 +633,17 @@ struct ChiKernel {
     double w;
     // G(v - ω/2) G(v + ω/2) dv/dx at the compactified coordinate x (and the same at y): the factors
     // that depend on one coordinate only
-    __device__ R gfac(double x) const {
-        const R v = (R)((2.0 * x - 1.0) / ((1.0 - x) * x));
+    __device__ R gfac(double x, R& v) const {
+        v = (R)((2.0 * x - 1.0) / ((1.0 - x) * x));
         const R dv = (R)((2.0 * x * x - 2.0 * x + 1) / ((1.0 - x) * (1.0 - x) * x * x));
         const R wr = (R)w, h = (R)0.5;
         const R Lam = (R)A.Lam;
         return G_full(M, A.L.Nsig, a, Lam, v - h * wr) * G_full(M, A.L.Nsig, a, Lam, v + h * wr) * dv;
     }
-    __device__ double operator()(double x, double y) const { return (double)(core(x, y) * gfac(x) * gfac(y)); }
-    // the vertex part of the integrand; the integrand is (core * gfac(x)) * gfac(y)
-    __device__ R core(double x, double y) const {
+    // the vertex part of the integrand at the frequencies v(x), v(y); the integrand is
+    // (core * gfac(x)) * gfac(y)
+    __device__ R core(R v, R vp) const {
         const Layout& L = A.L;
-        const R v = (R)((2.0 * x - 1.0) / ((1.0 - x) * x));
-        const R vp = (R)((2.0 * y - 1.0) / ((1.0 - y) * y));
         const R wr = (R)w, h = (R)0.5;
         Plan<R> p1[3];
         make_plan<R>(p1[0], 0, v + vp, h * (v - wr - vp), h * (-v - wr + vp), M, L.Ns, L.NO, L.Nn);
@@ -756,32 +755,48 @@ struct ChiKernelFF {
     }
 };
 
-// evaluate regions reg(e) of one integral, e in [0, count), the block taking every CL-th
-// chunk of kChiChunk regions from chunk `first`: the 17 points of a chunk over all threads,
-// then each region's rule; emit(e, r, err) sees every result.  Region records are read
-// through L2 (other blocks of the cluster write them).
+// evaluate regions reg(e) of one integral, e in [0, count), which are the one first region or the halves of
+// cut regions in pairs, the block taking every `stride`-th chunk of regions from chunk `first`: the 17
+// points of a chunk over all threads, then each region's rule; emit(e, r, err) sees every result.  Region
+// records are read through L2 (other blocks of the cluster write them).  Rounds of few regions are cut into
+// smaller chunks, so that every block of a cluster has one.
 template <class F, class Reg, class Emit>
 __device__ void chi_eval_block(const F& f, const ChiRegions& R, const Reg& reg, int count, int first, int stride,
                                ChiScratch& S, const Emit& emit) {
     const int tid = threadIdx.x;
-    for (int cb = first * kChiChunk; cb < count; cb += stride * kChiChunk) {
-        const int cnt = min(kChiChunk, count - cb);
+    const int chunk = min(kChiChunk, (count + 2 * stride - 1) / (2 * stride) * 2);
+    for (int cb = first * chunk; cb < count; cb += stride * chunk) {
+        const int cnt = min(chunk, count - cb);
         if constexpr (F::kSplit) {
-            // the propagator factors depend on one coordinate: seven per axis and region instead of
-            // four per point (the integrand is (core(x, y) gfac(x)) gfac(y) either way)
-            for (int p = tid; p < cnt * 14; p += kChiThreads) {
-                const int r = reg(cb + p / 14), j = p % 14;
-                S.gfac[p] = j < 7 ? f.gfac(gm_coord(j, __ldcg(R.c0 + r), __ldcg(R.h0 + r)))
-                                  : f.gfac(gm_coord(j - 7, __ldcg(R.c1 + r), __ldcg(R.h1 + r)));
+            // What depends on one coordinate is computed for the seven coordinates per axis of a region, not for
+            // every point (the integrand is (core(x, y) gfac(x)) gfac(y) either way), and the two halves of a cut
+            // region share the axis that was not cut: 21 evaluations for a pair of regions.  (FP64 operations
+            // bound this: with the frequencies computed at every point and 28 factors per pair a call at
+            // Λ = 4 on square L = 4 took 427 ms.)
+            const int items = count == 1 ? 14 : cnt / 2 * 21;
+            for (int p = tid; p < items; p += kChiThreads) {
+                int q = p / 21 * 2, j = p - p / 21 * 21;
+                if (j >= 14) {  // the second half: its cut axis
+                    const bool x_shared = __ldcg(R.c0 + reg(cb + q)) == __ldcg(R.c0 + reg(cb + q + 1));
+                    ++q;
+                    j -= x_shared ? 7 : 14;
+                }
+                const int r = reg(cb + q);
+                S.gfac[14 * q + j] = j < 7 ? f.gfac(gm_coord(j, __ldcg(R.c0 + r), __ldcg(R.h0 + r)), S.freq[14 * q + j])
+                                           : f.gfac(gm_coord(j - 7, __ldcg(R.c1 + r), __ldcg(R.h1 + r)), S.freq[14 * q + j]);
             }
             __syncthreads();
             for (int p = tid; p < cnt * 17; p += kChiThreads) {
-                const int q = p / 17, r = reg(cb + q);
+                const int q = p / 17;
                 int xi, yi;
-                gm_index(p % 17, xi, yi);
-                const double x = gm_coord(xi, __ldcg(R.c0 + r), __ldcg(R.h0 + r));
-                const double y = gm_coord(yi, __ldcg(R.c1 + r), __ldcg(R.h1 + r));
-                S.f[p] = (double)(f.core(x, y) * S.gfac[14 * q + xi] * S.gfac[14 * q + 7 + yi]);
+                gm_index(p - 17 * q, xi, yi);
+                xi += 14 * q;
+                yi += 14 * q + 7;
+                if (q & 1) {
+                    if (__ldcg(R.c0 + reg(cb + q - 1)) == __ldcg(R.c0 + reg(cb + q))) xi -= 14;
+                    else yi -= 14;
+                }
+                S.f[p] = (double)(f.core(S.freq[xi], S.freq[yi]) * S.gfac[xi] * S.gfac[yi]);
             }
         } else {
             for (int p = tid; p < cnt * 17; p += kChiThreads) {

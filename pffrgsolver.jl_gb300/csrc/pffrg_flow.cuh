@@ -62,8 +62,17 @@ struct NodeScratch {
 // L = 6 two-loop state 32x2 teams with 4 nodes ran 403 ms against 470 ms with 8 nodes (two blocks
 // per SM instead of three), and 16x3 teams were slower with 1 node than with 2.
 template <int T, int C, int SPL>
+__host__ __device__ constexpr int base_batch() { return (C == 2 ? (SPL <= 4 ? 4 : 2) : 4) * T / 32; }
+// The setup runs the propagators of a batch first, then its plans, and a step of the warp that holds both
+// costs the sum of the two.  One-site SU(2) teams of 16 lanes, and of 8 in FP64, therefore take twice the
+// nodes: FP64 square L = 3 68 -> 58 ms (50/15/10, noise) and 3.8 -> 3.3 ms (11/4/3), a honeycomb L = 4
+// parquet solve 33.5 -> 30.7 ms, a mixed cubic L = 4 step 94 -> 90 ms.  Four times the nodes left one block
+// per SM (76 ms), FP32 teams of 8 lanes were 2 % slower with twice (8.6 against 8.45 ms), and 32 lanes
+// hold a batch's setup in one step already.  The chunks of a level keep base_batch as their least size.
+template <typename R, int T, int C, int SPL>
 struct BatchOf {
-    static constexpr int NB = (C == 2 ? (SPL <= 4 ? 4 : 2) : 4) * T / 32;
+    static constexpr bool twice = C == 2 && SPL == 1 && (T == 16 || (T == 8 && sizeof(R) == 8));
+    static constexpr int NB = (twice ? 2 : 1) * base_batch<T, C, SPL>();
 };
 
 // SU(2) t-channel staging: per site the NB (spin, density) pairs of a batch, padded by 16 bytes so
@@ -75,7 +84,7 @@ __host__ __device__ constexpr int t_site_stride() {
 
 template <typename R, int T, int C, int SPL>
 struct TeamScratch {
-    NodeScratch<R, C> node[BatchOf<T, C, SPL>::NB];
+    NodeScratch<R, C> node[BatchOf<R, T, C, SPL>::NB];
 };
 
 // ---------------------------------------------------------------------------
@@ -329,7 +338,7 @@ struct Team {
         const int Ns = A.L.Ns;
         const int nslots = (X == 1) ? 4 : 2;
         const bool kat = A.prop_kind == PROP_KAT;
-        const int nitems = 2 + 3 * nslots;
+        const int nplans = 3 * nslots, nitems = 2 + nplans;
         nodes += count;
         // teams of one warp may hold different channels and batch lengths: every lane runs
         // the same sequence of warp syncs, bounded by the warp's longest batch
@@ -340,11 +349,14 @@ struct Team {
         unsigned corners = 0;  // corners of this lane's plans times the sites that read them
 #pragma unroll 1
         for (int it = tl; it < count * nitems; it += T) {
-            const int j = it / nitems, item = it - j * nitems;
+            // the propagators of all nodes, then the plans
+            const int k = it - 2 * count;
+            const int j = k < 0 ? it >> 1 : k / nplans;
             NodeScratch<R, C>& ns = ts.node[j];
             const double xj = ns.x;
             const SetupT v = SetupT(xj);
-            if (item < 2) {
+            if (k < 0) {
+                const int item = it & 1;
                 if constexpr (sizeof(R) == 4)
                     ns.prop[item] = prop_term(kat, M, A.prop_a, A.prop_da, (float)A.Lam,
                                               prop_freq(X, item, v, FF{0.5f, 0.f} * W));
@@ -352,8 +364,7 @@ struct Team {
                     ns.prop[item] = prop_term(kat, M, A.prop_a64, A.prop_da64, A.pc, prop_freq(X, item, v, 0.5 * W));
                 continue;
             }
-            const int k = item - 2;
-            const int slot = k / 3, ch = k - 3 * slot;
+            const int sc = k - j * nplans, slot = sc / 3, ch = sc - 3 * slot;
             NodePlan<R>& P = ns.plan[slot][ch];
             if (!(A.mask[X][slot] & (1 << ch))) {
                 P.nc = 0;
@@ -527,7 +538,7 @@ struct Team {
     // shared memory and both slots staged as [site][node] (spin, density) pairs for the overlap sums
     template <class Sink>
     __device__ __forceinline__ void eval_su2_nodes(int X, int count, Sink& sink) {
-        constexpr int NB = BatchOf<T, C, SPL>::NB;
+        constexpr int NB = BatchOf<R, T, C, SPL>::NB;
         using R2 = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
         const int Ns = A.L.Ns;
         constexpr int SS = t_site_stride<R, NB>();
@@ -579,7 +590,7 @@ struct Team {
     // values whose sums are never used.
     template <class Sink>
     __device__ __forceinline__ void eval_t_overlap(int count, Sink& sink) {
-        constexpr int NB = BatchOf<T, C, SPL>::NB;
+        constexpr int NB = BatchOf<R, T, C, SPL>::NB;
         using R2 = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
         const int Ns = A.L.Ns;
         constexpr int SS = t_site_stride<R, NB>();
@@ -926,6 +937,7 @@ __host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, i
 // the SMs' FP64 pipes and caches; otherwise the warps of a block take neighbouring chunks, which share
 // vertex rows.
 constexpr int kSMs = 152;
+constexpr int kDeepWave = 10;  // levels of more than 2048 new nodes per subdomain
 __host__ __device__ inline int eval_blocks(int nchunks, int npw) {
     const int units = (nchunks + npw - 1) / npw;
     const int full = (units + kWarps - 1) / kWarps;
@@ -981,7 +993,7 @@ struct SmemLayout {
     // t-channel staging per team: SU(2) both slots, the overlap sums and the local parts of the
     // whole batch, U(1)-DM one node
     __host__ __device__ static size_t tmp_per_team(int Ns) {
-        return C == 2 ? (size_t)4 * Ns * t_site_stride<R, BatchOf<T, C, SPL>::NB>() + (size_t)4 * Ns * BatchOf<T, C, SPL>::NB
+        return C == 2 ? (size_t)4 * Ns * t_site_stride<R, BatchOf<R, T, C, SPL>::NB>() + (size_t)4 * Ns * BatchOf<R, T, C, SPL>::NB
                       : (size_t)2 * C * Ns;
     }
     // the meshes of the node setup: float-float pairs and inverse spacings (mixed path) or FP64
@@ -1188,7 +1200,7 @@ __global__ void __launch_bounds__(kWarps * 32, wave0_min_blocks<R, SPL, C>()) wa
     const int Ns = A.L.Ns;
     const int jobs = 4 * A.eval + 1;
     const long long nwarps = (long long)gridDim.x * kWarps;
-    constexpr int NB = BatchOf<T, C, SPL>::NB;
+    constexpr int NB = BatchOf<R, T, C, SPL>::NB;
     // the FP64 pass of the mixed path starts only the subdomains the FP32 pass handed to it
     const int nwork = A.esc_mode == 2 ? Wsp.counters[5] : Wsp.nsub;
     for (long long base = ((long long)blockIdx.x * kWarps + warp) * NPW; base < nwork; base += nwarps * NPW) {
@@ -1373,10 +1385,11 @@ template <typename R, int T, int SPL, int C>
 __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
     eval_kernel(PassArgs<R> A, WaveSpace Wsp, int par, long long n) {
     constexpr int NPW = 32 / T;
-    constexpr int NB = BatchOf<T, C, SPL>::NB;
+    constexpr int NB = BatchOf<R, T, C, SPL>::NB;
     extern __shared__ __align__(16) unsigned char smem[];
     const int nactive = Wsp.counters[2 + par];
-    const LevelCut K = cut_level(nactive, n, Wsp.qcap, NB, C == 6 ? 1 : NB, Wsp.teams);
+    const LevelCut K = cut_level(nactive, n, Wsp.qcap, base_batch<T, C, SPL>(),
+                                 C == 6 ? 1 : base_batch<T, C, SPL>(), Wsp.teams);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         // the next level's list starts empty (this wave's decide_kernel fills it)
         Wsp.counters[2 + (par ^ 1)] = 0;
@@ -1500,8 +1513,8 @@ __global__ void __launch_bounds__(kWarps * 32) decide_kernel(WaveSpace Wsp, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int team = lane / T, tl = lane % T;
     const int bteam = warp * NPW + team;
-    const LevelCut K = cut_level(Wsp.counters[2 + par], n, Wsp.qcap, BatchOf<T, C, SPL>::NB,
-                                 C == 6 ? 1 : BatchOf<T, C, SPL>::NB, Wsp.teams);
+    const LevelCut K = cut_level(Wsp.counters[2 + par], n, Wsp.qcap, base_batch<T, C, SPL>(),
+                                 C == 6 ? 1 : base_batch<T, C, SPL>(), Wsp.teams);
     const int* active = par ? Wsp.active[1] : Wsp.active[0];
     const bool split = K.chunks >= kDecideSplit;
     const int G = split ? TPB : 1, g = split ? bteam : 0;
@@ -1704,10 +1717,14 @@ struct PassLauncher {
             const int gd = std::max(1, std::min(grid_cap, (Wsp.nsub + teams_per_block - 1) / teams_per_block));
             int par = 1;
             for (int wave = 1; wave <= 21; ++wave) {
-                eval_kernel<R, T, SPL, C><<<grid_cap, kWarps * 32, smem, st>>>(a, Wsp, par, 2ll << wave);
+                // most states end before the deep levels, whose subdomains are few: smaller grids, which come and
+                // go in half the time (a block takes several chunks where there are more)
+                const bool deep = wave > kDeepWave;
+                eval_kernel<R, T, SPL, C><<<deep ? std::min(grid_cap, 8 * kSMs) : grid_cap, kWarps * 32, smem, st>>>(
+                    a, Wsp, par, 2ll << wave);
                 h_counters[7] += 2;
                 if ((e = cudaGetLastError())) return e;
-                decide_kernel<T, SPL, C><<<gd, kWarps * 32, 0, st>>>(Wsp, a.L.Ns, a.atol, a.rtol, par, 2ll << wave,
+                decide_kernel<T, SPL, C><<<deep ? std::min(gd, 2 * kSMs) : gd, kWarps * 32, 0, st>>>(Wsp, a.L.Ns, a.atol, a.rtol, par, 2ll << wave,
                                                                      a.esc_mode, a.esc_eps);
                 if ((e = cudaGetLastError())) return e;
                 par ^= 1;
@@ -1726,8 +1743,8 @@ struct PassLauncher {
             if ((e = cudaStreamSynchronize(st))) return e;
             const int nact = h_counters[2 + par];
             if (nact == 0) break;
-            const LevelCut K = cut_level(nact, 2ll << wave, Wsp.qcap, BatchOf<T, C, SPL>::NB,
-                                 C == 6 ? 1 : BatchOf<T, C, SPL>::NB, Wsp.teams);
+            const LevelCut K = cut_level(nact, 2ll << wave, Wsp.qcap, base_batch<T, C, SPL>(),
+                                 C == 6 ? 1 : base_batch<T, C, SPL>(), Wsp.teams);
             if (K.overflow) {  // chunk queue overflow
                 h_counters[4] = 1;
                 return cudaErrorLaunchOutOfResources;

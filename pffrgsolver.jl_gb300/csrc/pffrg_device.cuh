@@ -825,7 +825,7 @@ __device__ __forceinline__ PropTerm<double> prop_term(bool kat, const MeshD& M, 
     return o;
 }
 
-// FP32, float-float frequency: the operations of prop_half_ff's halves, each frequency once
+// FP32 at a float-float frequency (bubbles.jl:64-96), the operations in the order of S_single and G_full
 __device__ __forceinline__ PropTerm<float> prop_term(bool kat, const MeshFF& M, const float* __restrict__ Sig,
                                                      const float* __restrict__ dSig, float L, FF a) {
     PropTerm<float> o;
@@ -896,37 +896,6 @@ template <typename S>
 __device__ __forceinline__ S prop_freq(int X, int item, S v, S hW) {
     if (X == 0 && item == 1) return hW + (-v);
     return v + ((X == 2) == (item == 1) ? hW : -hW);
-}
-
-// prop_half with float-float frequencies (bubbles.jl:64-96)
-__device__ __forceinline__ float prop_half_ff(int kind, int half, int ch, const MeshFF& M, int Nsig, const float* Sig,
-                                              const float* dSig, float L, FF v, FF W) {
-    const FF hW = FF{0.5f, 0.f} * W;
-    FF w1, w2;
-    if (ch == 0) {
-        w1 = v + hW;
-        w2 = hW - v;
-    } else if (ch == 1) {
-        w1 = v + hW;
-        w2 = v - hW;
-    } else {
-        w1 = v - hW;
-        w2 = v + hW;
-    }
-    if (kind == 0) {  // get_propagator_kat: (S(a) + G(a)^2 dΣ(a)) G(b)
-        const FF a = half == 0 ? w1 : w2, b = half == 0 ? w2 : w1;
-        float ds = 0.f;
-        const float sa = get_sigma_ff(M, Nsig, Sig, a, dSig, &ds);
-        const float g1 = G_full_s(sa, L, a.h);
-        const float g0 = G_bare(L, a.h);
-        const float r = g1 / g0;
-        const float s1 = fabsf(a.h) > 1e-8f ? r * r * expf(-(a.h * a.h) / (L * L)) * 2.f * a.h / (L * L * L) : 0.f;
-        const float g2 = G_full_s(get_sigma_ff(M, Nsig, Sig, b), L, b.h);
-        return (s1 + g1 * g1 * ds) * g2 / two_pi<float>();
-    }
-    const float g1 = G_full_s(get_sigma_ff(M, Nsig, Sig, w1), L, w1.h);
-    const float g2 = G_full_s(get_sigma_ff(M, Nsig, Sig, w2), L, w2.h);
-    return -(g1 * g2) / two_pi<float>();
 }
 
 }  // namespace pffrg

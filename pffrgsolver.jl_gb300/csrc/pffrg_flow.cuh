@@ -50,6 +50,12 @@ constexpr int kWarps = 4;
 template <typename R, int C>
 struct NodeScratch {
     double x;      // the node (integration variable v)
+    // the node as the setup uses it: converting it costs FP64 operations, once per node instead of at every step
+    typename std::conditional<sizeof(R) == 4, FF, double>::type xs;
+    __device__ __forceinline__ void set(double v) {
+        x = v;
+        xs = decltype(xs)(v);
+    }
     PropTerm<R> prop[2];
     R p;           // the bubble propagator
     R loc[2 * C];  // t channel: local vertices v3[C], v4[C] at site 1
@@ -353,8 +359,7 @@ struct Team {
             const int k = it - 2 * count;
             const int j = k < 0 ? it >> 1 : k / nplans;
             NodeScratch<R, C>& ns = ts.node[j];
-            const double xj = ns.x;
-            const SetupT v = SetupT(xj);
+            const SetupT v = ns.xs;
             if (k < 0) {
                 const int item = it & 1;
                 if constexpr (sizeof(R) == 4)
@@ -381,7 +386,7 @@ struct Team {
                 if (ff_near_switch(a0, scale, M, A.L.NO, A.L.Nn) || ff_near_switch(a1, scale, M, A.L.NO, A.L.Nn) ||
                     ff_near_switch(a2, scale, M, A.L.NO, A.L.Nn))
                     kernel = plan_fp64(P, A.mesh, A.L.Nsig, A.L.NO, A.L.Nn, Ns, q0(), X, ti.w1, (slot & 1) ? ti.w3 : ti.w2,
-                                       ch, code, xj);
+                                       ch, code, ns.x);
                 else
                     kernel = build_plan(P, ch, a0, a1, a2, M, Ns, q0());
             } else {
@@ -1258,7 +1263,7 @@ __global__ void __launch_bounds__(kWarps * 32, wave0_min_blocks<R, SPL, C>()) wa
 #pragma unroll 1
         for (int b = 0; b < 5; b += NB) {
             const int nb = max(0, min(NB, cnt - b));
-            for (int j = tl; j < nb; j += T) tm.ts.node[j].x = x[b + j];
+            for (int j = tl; j < nb; j += T) tm.ts.node[j].set(x[b + j]);
             __syncwarp();
             auto add = [&](int j, const R (&gv)[C][SPL]) {
                 const int q = b + j;
@@ -1455,7 +1460,7 @@ __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
             const int nb = max(0, min(NB, cnt - b));
             if (tl < nb) {
                 const int nd = first + b + tl;  // 0-based new node of the level
-                tm.ts.node[tl].x = sgn * __dadd_rn(lo, __dmul_rn(2.0 * (double)(nd + 1) - 1.0, h));
+                tm.ts.node[tl].set(sgn * __dadd_rn(lo, __dmul_rn(2.0 * (double)(nd + 1) - 1.0, h)));
             }
             __syncwarp();
             tm.eval(ti, W, V, VP, nb, add);

@@ -775,8 +775,16 @@ struct PropTerm {
 
 // constants of the regulator exp(-w²/Λ²)
 struct PropConst {
-    double L2, iL2, twoL3;  // Λ², 1/Λ², 2/Λ³
+    double L2, iL2, twoL3;  // Λ², 1/Λ², 2/Λ³ (prop_const)
 };
+
+// The single-scale factor exp(-w²/Λ²) 2 w/Λ³ is zero at every |w| > 1e-8 long before 2/Λ³ overflows
+// (Λ < 2.2e-103), and has to stay so: 0 times an infinite factor would be NaN.  Any bound that no Λ with a
+// nonzero exponential reaches serves (Λ = 1e-66 at 1e200).
+inline PropConst prop_const(double L) {
+    const double L2 = L * L, L3 = L * L * L, t = 2.0 / L3;
+    return PropConst{L2, 1.0 / L2, L3 > 0.0 && t > 1e200 ? 1e200 : t};
+}
 
 // FP64: with E = 1 - exp(-w²/Λ²), G0 = E/w, G = E/(w + E Σ) and G/G0 = w/(w + E Σ) share one
 // reciprocal; Σ and dΣ share one interval search.  About 50 FP64 operations for a frequency; prop_half's
@@ -809,7 +817,8 @@ __device__ __forceinline__ PropTerm<double> prop_term(bool kat, const MeshD& M, 
     const double w2 = w * w;
     double x = w2 * c.iL2;
     x = fma(fma(-x, c.L2, w2), c.iL2, x);
-    if ((__double2hiint(c.iL2) & 0x7ff00000) >= 0x7fe00000) x = w2 / c.L2;  // Λ² at or near zero
+    // the product, its correction or 1/Λ² left the range (Λ² at or near zero or infinite, w/Λ above 1e154)
+    if ((__double2hiint(x) & 0x7ff00000) == 0x7ff00000) x = w2 / c.L2;
     double ex, em1;
     exp_and_m1(-x, ex, em1);
     // a Σ of the other sign than w is left out (G_full)

@@ -1693,8 +1693,7 @@ struct PassLauncher {
         // blocks (three for FP64) still fits on an SM (228 KB less 1 KB per block; a row word is read
         // once per batch of nodes, so from L1 it costs little)
         PassArgs<R> a = a0;
-        const double L2 = a.Lam * a.Lam;
-        a.pc = PropConst{L2, 1.0 / L2, 2.0 / (a.Lam * a.Lam * a.Lam)};
+        a.pc = prop_const(a.Lam);
         const int nm = a.L.Nsig + 2 * a.L.NO + 2 * a.L.Nn;
         const size_t staged = SmemLayout<R, T, C, SPL>(a.L.Ns, nm, a.rows_total, true).total;
         constexpr int fit_kb = 228 / (sizeof(R) == 4 ? eval_min_blocks<R, T, SPL, C>() : 3) - 1;

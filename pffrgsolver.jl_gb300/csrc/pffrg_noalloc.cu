@@ -177,9 +177,11 @@ int pffrg_dgamma_1l_noalloc(const pffrg_lattice_view* lat, const pffrg_mesh_view
     o = align_up(o + sizeof(int));
     const size_t o_wave = o;
     o += wave_space_bytes(nsub, Ns, qcap, 2);
-    // chunk records of two levels, which the passes no longer keep: counted so that the problems this
-    // entry point takes and refuses stay the same
-    o += 2 * align256(sizeof(int4) * qcap);
+    // The entry point takes and refuses the problems it always did: counted are subdomain records of 56 bytes
+    // and chunk records of two levels, which the passes no longer keep.
+    constexpr size_t kCountedRecord = 56;
+    static_assert(sizeof(SubRec) <= kCountedRecord, "the count covers the records kept");
+    o += align256(kCountedRecord * nsub) - align256(sizeof(SubRec) * nsub) + 2 * align256(sizeof(int4) * qcap);
     if (o > kNoAllocScratchBytes)
         return fail(PFFRG_E_LIMIT,
                     "problem needs %zu bytes of scratch, the no-allocation entry point holds %zu "

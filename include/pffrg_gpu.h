@@ -266,8 +266,8 @@ int64_t pffrg_last_integrand_evals(const pffrg_ctx* ctx);
 /* Work counters and optional CUDA-event timing (recorded on the context's stream). */
 typedef struct pffrg_stats {
     int64_t integrand_evals;    /* bubble integrand evaluations of the last RHS / dΓ call */
-    int64_t algorithmic_values; /* vertex values those evaluations read (corners x sites x components,
-                                   bare and output values, t-channel overlap operands) */
+    int64_t algorithmic_values; /* vertex values those evaluations read (corners of nonzero weight x sites x
+                                   components, bare and output values, t-channel overlap operands) */
     double pass_ms;             /* summed duration of the channel-task kernels since the last reset */
     double rhs_ms;              /* summed duration of pffrg_rhs calls since the last reset */
     int64_t pass_launches;      /* channel-task passes (each a sequence of level kernels) since the last reset */

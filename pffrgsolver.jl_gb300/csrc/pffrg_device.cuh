@@ -315,10 +315,6 @@ __device__ __forceinline__ int comp_read(const PL& P, int C, int c, R& sgn) {
     return src;
 }
 
-__host__ __device__ constexpr int corners_of(int kernel) {
-    return kernel == 0 ? 0 : (kernel == 1 ? 2 : (kernel == 4 ? 8 : 4));
-}
-
 // ---------------------------------------------------------------------------
 // self energy and propagators
 // ---------------------------------------------------------------------------
@@ -673,10 +669,10 @@ __device__ __forceinline__ Param<double> find(double x, const MeshD& M, int o, i
 // The plan of one buffer (same sign folding, kernel choice and corner order as make_plan).  Corners
 // of an argument that lies exactly on a mesh point, whose second weight is zero, are left out: the
 // bubbles read their own channel at the task's mesh frequencies, where two corners of eight remain.
-// q0: offset of the first kernel of the s channel.  Returns the kernel (0 none, 1 q1, ..., 4 q3).
+// q0: offset of the first kernel of the s channel.
 template <typename R, typename S, typename MV>
-__device__ __forceinline__ int build_plan(NodePlan<R>& P, int chan, S w, S v, S vp, const MV& M, int Ns,
-                                          int64_t q0) {
+__device__ __forceinline__ void build_plan(NodePlan<R>& P, int chan, S w, S v, S vp, const MV& M, int Ns,
+                                           int64_t q0) {
     const bool nw = is_neg(w), nv = is_neg(v), np = is_neg(vp);
     if (nw) w = -w;
     if (nv) v = -v;
@@ -692,11 +688,11 @@ __device__ __forceinline__ int build_plan(NodePlan<R>& P, int chan, S w, S v, S 
     const int on = chan == 1 ? M.nt() : M.ns();
     if (beyond(M.at(oO, NO - 1), w)) {  // get_buffer (buffer.jl:51-84): beyond the bosonic mesh
         P.nc = 0;
-        return 0;
+        return;
     }
     const S last = M.at(on, Nn - 1);
     const bool vin = !beyond(last, v), vpin = !beyond(last, vp);
-    const int kernel = vin ? (vpin ? 4 : 2) : (vpin ? 3 : 1);
+    const int kernel = vin ? (vpin ? 4 : 2) : (vpin ? 3 : 1);  // q1, q2_1, q2_2, q3
     const int src_ch = (chan == 1) ? 1 : ((chan == 0) == mp ? 2 : 0);
     P.exch = ex ? 1 : 0;
     P.flags = (smn ? 1 : 0) | (sm ? 2 : 0) | (sn ? 4 : 0);
@@ -726,7 +722,6 @@ __device__ __forceinline__ int build_plan(NodePlan<R>& P, int chan, S w, S v, S 
         }
     }
     P.nc = n;
-    return kernel;
 }
 
 // exp(x) and exp(x) - 1 for x <= 0, within an ulp of each.  x = k ln 2 + r with |r| <= ln(2)/2, the

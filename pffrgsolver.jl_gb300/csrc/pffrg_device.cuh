@@ -669,10 +669,10 @@ __device__ __forceinline__ Param<double> find(double x, const MeshD& M, int o, i
 // The plan of one buffer (same sign folding, kernel choice and corner order as make_plan).  Corners
 // of an argument that lies exactly on a mesh point, whose second weight is zero, are left out: the
 // bubbles read their own channel at the task's mesh frequencies, where two corners of eight remain.
-// q0: offset of the first kernel of the s channel.
+// q0: offset of the first kernel of the s channel.  Returns the number of corners.
 template <typename R, typename S, typename MV>
-__device__ __forceinline__ void build_plan(NodePlan<R>& P, int chan, S w, S v, S vp, const MV& M, int Ns,
-                                           int64_t q0) {
+__device__ __forceinline__ int build_plan(NodePlan<R>& P, int chan, S w, S v, S vp, const MV& M, int Ns,
+                                          int64_t q0) {
     const bool nw = is_neg(w), nv = is_neg(v), np = is_neg(vp);
     if (nw) w = -w;
     if (nv) v = -v;
@@ -688,7 +688,7 @@ __device__ __forceinline__ void build_plan(NodePlan<R>& P, int chan, S w, S v, S
     const int on = chan == 1 ? M.nt() : M.ns();
     if (beyond(M.at(oO, NO - 1), w)) {  // get_buffer (buffer.jl:51-84): beyond the bosonic mesh
         P.nc = 0;
-        return;
+        return 0;
     }
     const S last = M.at(on, Nn - 1);
     const bool vin = !beyond(last, v), vpin = !beyond(last, vp);
@@ -722,6 +722,7 @@ __device__ __forceinline__ void build_plan(NodePlan<R>& P, int chan, S w, S v, S
         }
     }
     P.nc = n;
+    return n;
 }
 
 // exp(x) and exp(x) - 1 for x <= 0, within an ulp of each.  x = k ln 2 + r with |r| <= ln(2)/2, the

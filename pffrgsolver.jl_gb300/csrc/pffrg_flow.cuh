@@ -303,13 +303,14 @@ __device__ __forceinline__ TaskInfo task_of(const PassArgs<R>& A, int sub, int j
 // The plan of a mixed-path argument near a buffer switch: the FP64 path's rounding decides the side.
 // Not inlined (and given values, not the kernel's arguments, whose address would copy them to local
 // memory): few lanes take it, and the kernels' code has to fit the instruction caches.
-static __device__ __noinline__ void plan_fp64(NodePlan<float>& P, const double* mesh, int Nsig, int NO, int Nn, int Ns,
-                                              int64_t q0, int X, int w1, int wf, int ch, unsigned code,
-                                              double x) {
+static __device__ __noinline__ int plan_fp64(NodePlan<float>& P, const double* mesh, int Nsig, int NO, int Nn, int Ns,
+                                             int64_t q0, int X, int w1, int wf, int ch, unsigned code,
+                                             double x) {
     const MeshD M = mesh_view_d(mesh, Nsig, NO, Nn);
     const double W = M.at(X == 1 ? M.Ot() : M.Os(), w1);
     const double F = wf >= 0 ? M.at(X == 1 ? M.nt() : M.ns(), wf) : INFINITY;
-    build_plan(P, ch, plan_arg(code, W, x, F), plan_arg(code >> 7, W, x, F), plan_arg(code >> 14, W, x, F), M, Ns, q0);
+    return build_plan(P, ch, plan_arg(code, W, x, F), plan_arg(code >> 7, W, x, F), plan_arg(code >> 14, W, x, F), M, Ns,
+                      q0);
 }
 
 template <typename R, int T, int SPL, int C>
@@ -378,19 +379,20 @@ struct Team {
             const SetupT F = (slot & 1) ? VP : V;
             const SetupT a0 = plan_arg(code, W, v, F), a1 = plan_arg(code >> 7, W, v, F),
                          a2 = plan_arg(code >> 14, W, v, F);
+            int nc;
             if constexpr (sizeof(R) == 4) {
                 const float scale = fabsf(v.h) + fabsf(W.h) + (isinf(V.h) ? 0.f : fabsf(V.h)) +
                                     (isinf(VP.h) ? 0.f : fabsf(VP.h));
                 if (ff_near_switch(a0, scale, M, A.L.NO, A.L.Nn) || ff_near_switch(a1, scale, M, A.L.NO, A.L.Nn) ||
                     ff_near_switch(a2, scale, M, A.L.NO, A.L.Nn))
-                    plan_fp64(P, A.mesh, A.L.Nsig, A.L.NO, A.L.Nn, Ns, q0(), X, ti.w1, (slot & 1) ? ti.w3 : ti.w2, ch, code,
-                              ns.x);
+                    nc = plan_fp64(P, A.mesh, A.L.Nsig, A.L.NO, A.L.Nn, Ns, q0(), X, ti.w1, (slot & 1) ? ti.w3 : ti.w2, ch,
+                                   code, ns.x);
                 else
-                    build_plan(P, ch, a0, a1, a2, M, Ns, q0());
+                    nc = build_plan(P, ch, a0, a1, a2, M, Ns, q0());
             } else {
-                build_plan(P, ch, a0, a1, a2, M, Ns, q0());
+                nc = build_plan(P, ch, a0, a1, a2, M, Ns, q0());
             }
-            corners += P.nc * (slot < 2 ? Ns : 1);
+            corners += nc * (slot < 2 ? Ns : 1);
         }
         if (A.node_counter) {
             alg += (unsigned long long)corners * C;

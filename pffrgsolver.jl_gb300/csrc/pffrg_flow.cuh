@@ -609,7 +609,7 @@ struct Team {
         // FP32 teams of a warp fetch the next row while one is worked on, across the end of a site's list too:
         // long lists do not fit in shared memory beside the staging and are read through L1, of which the
         // vertex gathers leave little (pyrochlore L = 6 two loops mixed 249 -> 235 ms; narrower teams, whose
-        // short lists stay in shared memory, were 1.5 % slower with it).
+        // short lists are staged in shared memory up to 14 sites, were 1.5 % slower with it).
         constexpr bool kAhead = sizeof(R) == 4 && T == 32;
         int r = tl, j1 = row_off[0], rn = j1 + tl;
         const int last = row_off[Ns] - 1;
@@ -1379,12 +1379,15 @@ __global__ void __launch_bounds__(kWarps * 32, wave0_min_blocks<R, SPL, C>()) wa
 }
 
 // ---- wave k >= 1: evaluate queued chunks, one partial node sum per chunk ----
-// (FP32 kernels: SU(2) teams with one site per lane held to 102 registers, five blocks of 128 threads per SM
-// (four, five and six blocks 11.0, 10.5 and 10.8 ms summed over two square L = 3 right-hand sides), with two
-// sites to 128, four blocks (their gathers spill beyond that); wider lanes and U(1)-DM entries, whose gathers
-// spill at 128, to 168, three blocks)
+// (FP32 kernels: SU(2) teams of 8 and 32 lanes with one site per lane held to 102 registers, five blocks of 128
+// threads per SM (four, five and six blocks 11.0, 10.5 and 10.8 ms summed over two square L = 3 right-hand
+// sides, 8 lanes); those of 16 lanes, whose blocks of 48 to 59 KB fit four times at most, and those with two
+// sites per lane to 128, four blocks (the latter's gathers spill beyond that); wider lanes and U(1)-DM entries,
+// whose gathers spill at 128, to 168, three blocks)
 template <typename R, int T, int SPL, int C>
-constexpr int eval_min_blocks() { return sizeof(R) == 4 ? (C == 2 && SPL <= 2 ? (SPL == 1 ? 5 : 4) : 3) : 1; }
+constexpr int eval_min_blocks() {
+    return sizeof(R) == 4 ? (C == 2 && SPL <= 2 ? (SPL == 1 && T != 16 ? 5 : 4) : 3) : 1;
+}
 
 template <typename R, int T, int SPL, int C>
 __global__ void __launch_bounds__(kWarps * 32, eval_min_blocks<R, T, SPL, C>())
@@ -1684,20 +1687,34 @@ inline cudaError_t allow_max_dynamic_smem() {
     return e;
 }
 
+// Whether a block's overlap rows are staged in shared memory (mode 1 never, 2 where they fit at all): by
+// default only while the FP32 eval kernel's register-bound number of blocks (three for FP64) still fits on an
+// SM, 228 KB less 1 KB per block; a row word is read once per batch of nodes, so from L1 it costs little.
+// FP32 teams of 16 lanes, whose batch scratch alone leaves three or four blocks, stage their rows while that
+// costs none of them: right-hand sides on 11 to 16 sites run 1 to 3 % faster than with a register cap for
+// five blocks and the rows in L1 (honeycomb L = 5 12.68 -> 12.29 ms, square L = 6 17.36 -> 16.96 ms, cubic
+// L = 5 19.34 -> 18.88 ms).  Their FP64 blocks of 73 to 91 KB don't: two or three fit either way, and staged
+// rows changed 11 to 16 sites by under 1 % and kagome L = 4 (13 sites) from 25.1 to 26.0 ms.
+template <typename R, int T, int C, int SPL>
+inline bool stage_rows(int Ns, int nm, long long rows, int mode) {
+    if (mode == 1) return false;
+    const size_t staged = SmemLayout<R, T, C, SPL>(Ns, nm, rows, true).total;
+    if (mode == 2) return staged <= (size_t)227 * 1024;
+    int blocks = sizeof(R) == 4 ? eval_min_blocks<R, T, SPL, C>() : 3;
+    if (sizeof(R) == 4 && BatchOf<R, T, C, SPL>::twice)
+        blocks = std::min(blocks, (int)((size_t)228 * 1024 / (SmemLayout<R, T, C, SPL>(Ns, nm, rows, false).total + 1024)));
+    return staged <= (size_t)(228 / blocks - 1) * 1024;
+}
+
 // team width T = lanes per node batch, SPL = sites per lane
 template <typename R, int C>
 struct PassLauncher {
     template <int T, int SPL>
     static cudaError_t run(const PassArgs<R>& a0, WaveSpace& Wsp, int* h_counters, cudaStream_t st, int grid_cap) {
-        // overlap rows in shared memory only while the FP32 eval kernel's register-bound number of
-        // blocks (three for FP64) still fits on an SM (228 KB less 1 KB per block; a row word is read
-        // once per batch of nodes, so from L1 it costs little)
         PassArgs<R> a = a0;
         a.pc = prop_const(a.Lam);
         const int nm = a.L.Nsig + 2 * a.L.NO + 2 * a.L.Nn;
-        const size_t staged = SmemLayout<R, T, C, SPL>(a.L.Ns, nm, a.rows_total, true).total;
-        constexpr int fit_kb = 228 / (sizeof(R) == 4 ? eval_min_blocks<R, T, SPL, C>() : 3) - 1;
-        a.rows_in_smem = a.rows_mode == 1 ? 0 : (staged <= (size_t)(a.rows_mode == 2 ? 227 : fit_kb) * 1024);
+        a.rows_in_smem = stage_rows<R, T, C, SPL>(a.L.Ns, nm, a.rows_total, a.rows_mode);
         SmemLayout<R, T, C, SPL> lay(a.L.Ns, nm, a.rows_total, a.rows_in_smem);
         const size_t smem = lay.total;
         if (smem > (size_t)227 * 1024) return cudaErrorInvalidConfiguration;

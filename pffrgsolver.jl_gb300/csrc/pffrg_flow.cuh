@@ -27,7 +27,7 @@
 // re-evaluating the integrand there.  Results are deterministic (fixed
 // summation order) and agree with the reference's arithmetic up to rounding.
 //
-// Node evaluation: a team of T lanes evaluates a batch of up to kBatch nodes.
+// Node evaluation: a team of T lanes evaluates a batch of up to BatchOf::NB nodes.
 // The lanes first split the batch's scalar work (propagator halves,
 // bubbles.jl; 6 or 12 interpolation plans, buffer.jl + channel.jl), then each
 // lane gathers and combines the vertex on its sites (flow_su2_{s,t,u}.jl,
@@ -180,7 +180,8 @@ __device__ __forceinline__ R gather_one(const PassArgs<R>& A, const NodeScratch<
         R acc;
         if constexpr (sizeof(R) == 4 && C == 6) {
             // the second product of a bosonic pair is rounded first: the FP32 results stay those of the
-            // uncompacted plan, in which the compiler chose this order (either is as exact)
+            // uncompacted plan, in which the compiler chose this order.  Either is as exact, but one chain of
+            // multiply-adds moves mixed right-hand sides of kagome L = 2 to 8 by 2e-9 to 5e-9 of their norm.
             int k = 1;
             acc = mul_rn(P.w[0], ldg(q + P.off[0] + st));
             if (P.flags & 8) {
@@ -823,8 +824,10 @@ struct Team {
                         x[5] = terms(p1.w, q2.y, q1.y, p2.y);
                     };
                     // refining nodes of lattices with three sites per lane: the first of an odd number of rows is
-                    // fused with the local part's factor, as a compiler unrolled these loops once; either order is
-                    // as exact, and FP32 results stay what they were
+                    // fused with the local part's factor, as a compiler unrolled these loops once, and the first
+                    // level and other lane widths are not.  It costs nothing measurable (kagome L = 8, 0.245 s
+                    // either way) and has no numerical purpose; without it such right-hand sides move by 3e-10
+                    // to 1.2e-9 of their norm, so it stays with the results.
                     const bool odd = odd_first && k < 2 && ((j1 - r) & 1);
                     if (odd) {
                         R x[C];
@@ -1560,8 +1563,9 @@ __global__ void __launch_bounds__(kWarps * 32) decide_kernel(WaveSpace Wsp, int 
             if (valid)
                 for (int q = q0; q < q1; ++q) fa_new += Wsp.part_abs[(size_t)a * K.chunks + q];  // triangle bound
         } else if (esc_mode == 1) {
-            // the norms of the coarse chunks, from the sums of their fine chunks: the bound (and with it
-            // which subdomains are handed off) does not depend on how a level was cut
+            // the norms of the coarse chunks, from the sums of their fine chunks: up to the FP32 rounding of
+            // these sums the bound does not depend on how a level was cut, so a finer cut can hand off another
+            // subdomain only where the bound meets the margin within that rounding
             const int r = K.chunks / K.coarse;
             const float* Q = fine_abs(Wsp, C * Ns) + (size_t)(valid ? a : 0) * K.chunks * C * Ns;
             for (int cc = 0; cc < ca; ++cc) {

@@ -725,10 +725,10 @@ __device__ __forceinline__ int build_plan(NodePlan<R>& P, int chan, S w, S v, S 
     return n;
 }
 
-// exp(x) and exp(x) - 1 for x <= 0, within an ulp of each.  x = k ln 2 + r with |r| <= ln(2)/2, the
-// Taylor sum of e^r - 1 to r^13 (the rest is below 1.2e-17 |r|) serves both: e^x - 1 = 2^k (e^r - 1) +
-// (2^k - 1), whose last bracket is exact.  23 FP64 operations instead of two library calls; largest error
-// seen on 2e7 arguments in (-700, 0): exp 0.86 ulp, exp - 1 0.90 ulp.
+// exp(x) and exp(x) - 1 for x <= 0, within an ulp of each.  x = k ln 2 + r with |r| <= ln(2)/2, reduced with
+// ln 2 in two parts (Cody and Waite 1980); the Taylor sum of e^r - 1 to r^13 (the rest is below 1.2e-17 |r|)
+// serves both: e^x - 1 = 2^k (e^r - 1) + (2^k - 1), whose last bracket is exact.  23 FP64 operations instead of
+// two library calls; largest error seen on 2e7 arguments in (-700, 0): exp 0.86 ulp, exp - 1 0.90 ulp.
 static __device__ __noinline__ double exp_far(double x) { return exp(x); }
 __device__ __forceinline__ void exp_and_m1(double x, double& ex, double& em1) {
     const double big = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer in the low bits

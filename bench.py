@@ -375,6 +375,8 @@ def ours(args):
         "gpu_launches": int(round(launches_step * args.steps)),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic,
+                     "frac_note": "vertex values read / time / copy peak: a normalised throughput, since they are read "
+                                  "from L1 and L2 (traffic: DRAM bytes); what bounds the kernels is under limiter",
                      "kernel": "quadrature wave kernels of the dΓ passes", "peak_kind": peak_kind,
                      "algorithmic_bytes_per_step": alg_bytes_step, "kernel_ms_per_step": pass_ms_step,
                      "launches_per_step": pass_launches_step,

@@ -787,8 +787,8 @@ inline PropConst prop_const(double L) {
 // chain of library calls and divisions, both halves of which evaluate both frequencies, takes over ten
 // times as many for the two.  The FP64 pipe (two operations per clock and SM) bounds the FP64 passes: with
 // this, integer comparisons, one argument formula for all lanes and the compacted plans, square L = 3
-// FP64 right-hand sides took 65 instead of 193 ms (50/15/10, noise) and 4.0 instead of 18.8 ms (11/4/3),
-// kagome L = 3 U(1)-DM 29 instead of 45 ms, pyrochlore L = 6 92 instead of 105 ms.
+// FP64 right-hand sides took 68 instead of 190 ms (50/15/10, noise) and 5.3 instead of 12.0 ms (11/4/3),
+// kagome L = 3 U(1)-DM 27 instead of 44 ms, pyrochlore L = 6 93 instead of 117 ms (means over three states).
 __device__ __forceinline__ PropTerm<double> prop_term(bool kat, const MeshD& M, const double* __restrict__ Sig,
                                                       const double* __restrict__ dSig, const PropConst& c, double w) {
     if (!(fabs(w) > 1e-8)) return PropTerm<double>{0.0, 0.0};

@@ -71,8 +71,8 @@ template <int T, int C, int SPL>
 __host__ __device__ constexpr int base_batch() { return (C == 2 ? (SPL <= 4 ? 4 : 2) : 4) * T / 32; }
 // The setup runs the propagators of a batch first, then its plans, and a step of the warp that holds both
 // costs the sum of the two.  One-site SU(2) teams of 16 lanes, and of 8 in FP64, therefore take twice the
-// nodes: FP64 square L = 3 68 -> 58 ms (50/15/10, noise) and 3.8 -> 3.3 ms (11/4/3), a honeycomb L = 4
-// parquet solve 33.5 -> 30.7 ms, a mixed cubic L = 4 step 94 -> 90 ms.  Four times the nodes left one block
+// nodes: FP64 square L = 3 68 -> 58 ms (50/15/10, noise) and 5.2 -> 4.5 ms (11/4/3), a honeycomb L = 4
+// parquet solve 33.9 -> 31.0 ms, a mixed cubic L = 4 step 94 -> 90 ms.  Four times the nodes left one block
 // per SM (76 ms), FP32 teams of 8 lanes were 2 % slower with twice (8.6 against 8.45 ms), and 32 lanes
 // hold a batch's setup in one step already.  The chunks of a level keep base_batch as their least size.
 template <typename R, int T, int C, int SPL>
@@ -913,9 +913,10 @@ struct LevelCut {
 // 8, 16 and 32 nodes; kagome L = 8 FP64: 10 ms for every level).  Chunks are therefore halved, down to one
 // batch of nodes, while the level still has fewer chunks than `teams`, about twice the teams that the GPU
 // holds at once; larger levels keep the coarse cut, whose partial sums cost least.  Right-hand sides and
-// steps, coarse cut only against this rule: square L = 3 11/4/3 FP64 40.1 -> 18.8 ms and 50/15/10 mixed
-// 34.1 -> 22.1 ms, kagome L = 8 U(1)-DM three loops mixed 482 -> 293 ms, honeycomb L = 5 two-loop step mixed
-// 222 -> 167 ms, pyrochlore L = 6 two loops mixed 377 -> 351 ms.
+// steps, coarse cut only against this rule, means over three states (the times of one case differ by up to a
+// factor of two between states): square L = 3 11/4/3 FP64 24.4 -> 12.0 ms and 50/15/10 mixed 30.7 -> 17.1 ms,
+// kagome L = 8 U(1)-DM three loops mixed 495 -> 304 ms, honeycomb L = 5 two-loop step mixed 222 -> 171 ms,
+// pyrochlore L = 6 two loops mixed 332 -> 302 ms.
 __host__ __device__ inline LevelCut cut_level(int nact, long long n, int qcap, int batch, int least, int teams) {
     LevelCut k;
     const int per0 = n <= (long long)kChunk * kMaxChunks ? (int)(n < kChunk ? n : kChunk) : (int)(n / kMaxChunks);

@@ -795,7 +795,7 @@ __device__ void chi_eval_block(const F& f, const ChiRegions& R, const Reg& reg, 
             // every point (the integrand is (core(x, y) gfac(x)) gfac(y) either way), and the two halves of a cut
             // region share the axis that was not cut: 21 evaluations for a pair of regions.  (FP64 operations
             // bound this: with the frequencies computed at every point and 28 factors per pair a call at
-            // Λ = 4 on square L = 4 took 427 ms, with this 383.)
+            // Λ = 4 on square L = 4 took 427 ms, with this 384.)
             const int items = count == 1 ? 14 : cnt / 2 * 21;
             for (int p = tid; p < items; p += kChiThreads) {
                 int q = p / 21 * 2, j = p - p / 21 * 21;
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(kChiThreads, 1) chi_box_kernel(ChiArgs A, cons
                     // stopping rule is the total error's): two lanes run them and leave every partial sum, and
                     // all threads test the rule, kChiThreads entries at a time.  (One thread that tested
                     // each entry as it went kept the other blocks of a cluster waiting: square L = 4 at
-                    // Λ = 4, 10 frequencies 383 against 302 ms with this.)
+                    // Λ = 4, 10 frequencies 384 against 303 ms with this, on the same state as above.)
                     for (int t0 = 0; t0 < nb; t0 += kChiThreads) {
                         const int nt = min(kChiThreads, nb - t0);
                         if (tid < 2) {
